@@ -542,10 +542,9 @@ class Engine : public HandleBase {
         for (int g = 0; g < nmat; ++g)
             for (int k = 0; k < 6; ++k) box[6 * g + k] = (k % 2) ? -1 : INT32_MAX;
         int* dbox = upload(box.data(), box.size());
-        const dim3 grd((nx + 255) / 256, ny, nz);
-        geometry_kernel<<<grd, 256, 0, st>>>(geom, layout(), ds, d->nshape, xs, ys, zs);
-        MFD_CK(cudaGetLastError());
-        geometry_box_kernel<<<grd, 256, 0, st>>>(geom, layout(), dbox);
+        const long long nblk = ((long long)ny * nz + GEO_TY - 1) / GEO_TY;
+        geometry_kernel<<<(unsigned)std::min(nblk, 148ll * 8), dim3(32, GEO_TY), 0, st>>>(geom, layout(), ds, d->nshape, xs, ys, zs,
+                                                                                        dbox, std::min(nmat, 255));
         MFD_CK(cudaGetLastError());
         MFD_CK(cudaMemcpyAsync(box.data(), dbox, box.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
         MFD_CK(cudaStreamSynchronize(st));

@@ -41,33 +41,65 @@ __host__ __device__ __forceinline__ bool shape_covers(const mfd_shape& s, double
     }
 }
 
-// One thread per cell of the padded map (x fastest); 1-D and 2-D grids take the missing
-// coordinates as 0 (2-D: y; 1-D: x and y).
-__global__ void __launch_bounds__(256) geometry_kernel(uint8_t* __restrict__ geom, const Layout L, const mfd_shape* __restrict__ shapes,
-                                                       const int nshape, const double* __restrict__ xs,
-                                                       const double* __restrict__ ys, const double* __restrict__ zs) {
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iy = blockIdx.y, iz = blockIdx.z;
-    if (ix >= L.nx) return;
-    const double x = xs ? xs[ix] : 0.0, y = ys ? ys[iy] : 0.0, z = zs[iz];
-    int g = 0;
-    for (int s = 0; s < nshape; ++s)
-        if (shape_covers(shapes[s], x, y, z)) g = shapes[s].material;
-    geom[ix + L.px * iy + (long long)L.sz * iz] = (uint8_t)g;
-}
+// The padded map (x fastest) and, in the same pass, the bounding box of each material's cells:
+// box[6 (g - 1) + {0..5}] = x0, x1, y0, y1, z0, z1 (initialised to INT_MAX / -1).  1-D and 2-D
+// grids take the missing coordinates as 0 (2-D: y; 1-D: x and y).
+//
+// A warp walks rows 32 cells at a time.  The lanes of one material are found with a ballot, so
+// a segment gives at most one candidate interval per material; it is merged into the block's
+// boxes in shared memory (an atomic only when it widens them, which soon becomes rare), and each
+// block merges its boxes into the global ones once.  What bounds it is the shapes' FP64 tests;
+// the six global atomics per material cell that a pass of its own took before were serialised
+// on six addresses per material (a 96 x 96 x 512 whole-domain glass: mfd_create 19.6 ms, now 2.6;
+// 32 2-D models of 128-1024 cells a side: 114 ms for their creation, now 26).
+constexpr int GEO_TY = 8;
 
-// Bounding box of each material's cells: box[6 (g - 1) + {0..5}] = x0, x1, y0, y1, z0, z1
-// (initialised to INT_MAX / -1).
-__global__ void __launch_bounds__(256) geometry_box_kernel(const uint8_t* __restrict__ geom, const Layout L, int* box) {
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iy = blockIdx.y, iz = blockIdx.z;
-    if (ix >= L.nx) return;
-    const int g = geom[ix + L.px * iy + (long long)L.sz * iz];
-    if (!g) return;
-    int* b = box + 6 * (g - 1);
-    atomicMin(b + 0, ix); atomicMax(b + 1, ix);
-    atomicMin(b + 2, iy); atomicMax(b + 3, iy);
-    atomicMin(b + 4, iz); atomicMax(b + 5, iz);
+__global__ void __launch_bounds__(32 * GEO_TY) geometry_kernel(uint8_t* __restrict__ geom, const Layout L,
+                                                               const mfd_shape* __restrict__ shapes, const int nshape,
+                                                               const double* __restrict__ xs, const double* __restrict__ ys,
+                                                               const double* __restrict__ zs, int* box, const int nmat) {
+    __shared__ int sb[6 * 255];
+    const int lane = threadIdx.x, tid = threadIdx.x + 32 * threadIdx.y;
+    for (int i = tid; i < 6 * nmat; i += 32 * GEO_TY) sb[i] = (i & 1) ? -1 : 0x7fffffff;
+    __syncthreads();
+    const long long rows = (long long)L.ny * L.nz;
+    for (long long row = (long long)blockIdx.x * GEO_TY + threadIdx.y; row < rows; row += (long long)gridDim.x * GEO_TY) {
+        const int iz = (int)(row / L.ny), iy = (int)(row - (long long)iz * L.ny);
+        const double y = ys ? ys[iy] : 0.0, z = zs[iz];
+        for (int x0 = 0; x0 < L.nx; x0 += 32) {
+            const int ix = x0 + lane;
+            int g = 0;
+            if (ix < L.nx) {
+                const double x = xs ? xs[ix] : 0.0;
+                for (int s = 0; s < nshape; ++s)
+                    if (shape_covers(shapes[s], x, y, z)) g = shapes[s].material;
+                g = (uint8_t)g;   // what the map holds
+                geom[ix + (long long)L.px * iy + (long long)L.sz * iz] = (uint8_t)g;
+            }
+            unsigned todo = __ballot_sync(0xffffffffu, g != 0);
+            while (todo) {
+                const int first = __ffs((int)todo) - 1;
+                const int gl = __shfl_sync(0xffffffffu, g, first);
+                const unsigned m = __ballot_sync(0xffffffffu, g == gl);
+                if (lane == first) {
+                    int* b = sb + 6 * (gl - 1);
+                    const int hi = x0 + 31 - __clz((int)m);
+                    if (ix < b[0]) atomicMin(b + 0, ix);
+                    if (hi > b[1]) atomicMax(b + 1, hi);
+                    if (iy < b[2]) atomicMin(b + 2, iy);
+                    if (iy > b[3]) atomicMax(b + 3, iy);
+                    if (iz < b[4]) atomicMin(b + 4, iz);
+                    if (iz > b[5]) atomicMax(b + 5, iz);
+                }
+                todo &= ~m;
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < 6 * nmat; i += 32 * GEO_TY) {
+        if (i & 1) { if (sb[i] >= 0) atomicMax(box + i, sb[i]); }
+        else if (sb[i] != 0x7fffffff) atomicMin(box + i, sb[i]);
+    }
 }
 
 }  // namespace mfd
