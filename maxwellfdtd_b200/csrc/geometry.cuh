@@ -50,8 +50,8 @@ __host__ __device__ __forceinline__ bool shape_covers(const mfd_shape& s, double
 // boxes in shared memory (an atomic only when it widens them, which soon becomes rare), and each
 // block merges its boxes into the global ones once.  What bounds it is the shapes' FP64 tests;
 // the six global atomics per material cell that a pass of its own took before were serialised
-// on six addresses per material (a 96 x 96 x 512 whole-domain glass: mfd_create 19.6 ms, now 2.6;
-// 32 2-D models of 128-1024 cells a side: 114 ms for their creation, now 26).
+// on six addresses per material (mfd_create of a 96 x 96 x 512 whole-domain glass: 19.6 ms
+// then, 1.1 now; of 1801 x 1203 cells with three materials: 2.2 ms then, 0.9 now).
 constexpr int GEO_TY = 8;
 
 __global__ void __launch_bounds__(32 * GEO_TY) geometry_kernel(uint8_t* __restrict__ geom, const Layout L,
