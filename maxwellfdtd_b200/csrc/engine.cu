@@ -302,6 +302,16 @@ static DivC<T> make_div(T d) {
         D.lob = a;
         D.span = b - a;
     }
+    if (sizeof(T) == 8 && d >= T(0x1p-300) && d <= T(0x1p300)) {   // high words of the band's ends
+        // powers of two, so that the high words bound the band exactly
+        const int e = std::ilogb(D.r) + 1;   // |r| < 2^e
+        const int lo = std::max(-900, -900 - e + 1), hi = std::min(900, 900 - e);
+        D.lo = (T)std::ldexp(1.0, lo);
+        D.hi = (T)std::ldexp(1.0, hi);
+        D.lob = (unsigned)(lo + 1023) << 20;
+        D.span = ((unsigned)(hi + 1023) << 20) - D.lob;
+        D.ok = 1;
+    }
     return D;
 }
 
@@ -314,6 +324,7 @@ class Engine : public HandleBase {
     int64_t nt = 0;
     T dx{}, dy{}, dz{}, dt{};
     DivC<T> ddx{}, ddy{}, ddz{};
+    bool kappa_one = true;       // every CPML kappa is 1 (the default)
     bool fastdiv = false;        // every divisor passed the device check
     bool recip = false;          // tolerance mode: derivatives by reciprocal multiply, fused multiply-adds
     Div3 d3{};                   // grid constants for the branch-free 3-D division (single precision)
@@ -577,10 +588,10 @@ class Engine : public HandleBase {
             std::vector<DivC<T>> dv = {make_div<T>(dx), make_div<T>(dy), make_div<T>(dz)};
             verify_divs(dv);
             ddx = dv[0]; ddy = dv[1]; ddz = dv[2];
-            fastdiv = sizeof(T) == 4 && ddx.ok && ddy.ok && ddz.ok;
-            if constexpr (sizeof(T) == 4) {   // band common to the three divisors (div6)
-                d3.dx = ddx.d; d3.dy = ddy.d; d3.dz = ddz.d;
-                d3.rx = ddx.r; d3.ry = ddy.r; d3.rz = ddz.r;
+            fastdiv = ddx.ok && ddy.ok && ddz.ok;
+            {   // band common to the three divisors (div6)
+                d3.dx = (float)ddx.d; d3.dy = (float)ddy.d; d3.dz = (float)ddz.d;   // single precision only
+                d3.rx = (float)ddx.r; d3.ry = (float)ddy.r; d3.rz = (float)ddz.r;
                 const unsigned lob = std::max(ddx.lob, std::max(ddy.lob, ddz.lob));
                 const unsigned hib = std::min(ddx.lob + ddx.span, std::min(ddy.lob + ddy.span, ddz.lob + ddz.span));
                 d3.lob1 = lob - 1u;
@@ -718,7 +729,10 @@ class Engine : public HandleBase {
                 std::vector<DivC<T>> kv;
                 for (int i = 0; i < L.nb; ++i) kv.push_back(make_div<T>((T)L.K[i]));
                 verify_divs(kv);
-                for (auto& D : kv) fastdiv = fastdiv && D.ok;
+                for (auto& D : kv) {
+                    fastdiv = fastdiv && D.ok;
+                    if (D.d != T(1)) kappa_one = false;
+                }
                 lay[f].K = upload(kv.data(), kv.size());
             }
             lay[f].A = upload_cast<T>(L.A, L.nb);
@@ -1454,6 +1468,16 @@ class Engine : public HandleBase {
     // DIV_RECIP in the tolerance mode, else DIV_EXACT when every divisor passed the device
     // check, else DIV_IEEE.
     template <typename F_>
+    void with_div1(F_&& f) {   // DIV_EXACT1 when every kappa is 1
+        if constexpr (sizeof(T) == 4) {
+            if (!recip && fastdiv && kappa_one) {
+                f(std::integral_constant<int, DIV_EXACT1>{});
+                return;
+            }
+        }
+        with_div(f);
+    }
+    template <typename F_>
     void with_div(F_&& f) {
         if (recip) f(std::integral_constant<int, DIV_RECIP>{});
         else if (fastdiv) f(std::integral_constant<int, DIV_EXACT>{});
@@ -1464,7 +1488,7 @@ class Engine : public HandleBase {
         HParams<T> p = hparams(accum, prev_step);
         if (ndim == 3 && use_split) {
             launch(KC_H, [&] {
-                with_div([&](auto dm) {
+                with_div1([&](auto dm) {
                     constexpr int D = decltype(dm)::value;
                     if (math_needed) launch_H_split_acc<true, D>(p);
                     else launch_H_split_acc<false, D>(p);
@@ -1514,7 +1538,7 @@ class Engine : public HandleBase {
         bool done = false;
         if (ndim == 3 && use_split) {
             launch(KC_E, [&] {
-                with_div([&](auto dm) {
+                with_div1([&](auto dm) {
                     constexpr int D = decltype(dm)::value;
                     if (any_geom) launch_E_split<true, D>(p, cur);
                     else launch_E_split<false, D>(p, cur);

@@ -48,8 +48,15 @@ struct Layout {
 // result equals RN(x/d) for every x in the band [lo, hi] (where they do) as soon as it does
 // for every significand of one binade.  The engine checks exactly that on the device, for
 // each divisor, against IEEE division over all 2^23 significands in [1, 2), and over the
-// band's lowest and highest binades, before the first step; a divisor that fails (or any
-// double-precision divisor) keeps IEEE division (ok = 0), as do numerators outside the band.
+// band's lowest and highest binades, before the first step; a divisor that fails keeps IEEE
+// division (ok = 0), as do numerators outside the band.
+//
+// Double precision cannot be checked exhaustively and takes the step twice (qcorr64 below).
+// With r = RN(1/d), q0 = RN(x r) is within 1.5 ulp of x/d; one step brings it within half an
+// ulp and a little more, so it is a faithful rounding; and for a faithful q and the correctly
+// rounded r, Markstein's theorem makes the next step RN(x/d) exactly, as long as nothing
+// underflows or overflows, which the band (2^-900 .. 2^900 for x and for the quotient)
+// ensures: the remainder x - q d is a multiple of 2^-1005 there.
 // Kernels take FAST = true only when every divisor of the model passed the check; the
 // band test is one unsigned compare on the bit pattern (lob = bits(lo), span = bits(hi) -
 // bits(lo)).  A zero numerator returns x (0/d keeps the sign of x since d > 0).
@@ -62,14 +69,17 @@ struct DivC {
 };
 
 // Division mode of a kernel (its FAST template parameter):
-//   DIV_IEEE  -- IEEE division (double precision, or a divisor that failed the check);
+//   DIV_IEEE  -- IEEE division (a divisor that failed the check or lies out of range);
 //   DIV_EXACT -- the verified correction step above, bit-identical to IEEE division;
 //   DIV_RECIP -- the tolerance mode: x * RN(1/d) (within an ulp of x/d), and the update
 //                expressions fused into multiply-adds (mad below) and the Poynting norm
 //                by the hardware reciprocal square root.  Results are no longer
 //                bit-identical to the reference's operation order; they stay within the
 //                relative L2 tolerance stated for the model's precision.
-enum { DIV_IEEE = 0, DIV_EXACT = 1, DIV_RECIP = 2 };
+//   DIV_EXACT1 -- DIV_EXACT for a model whose CPML kappas are all 1 (the default): the 3-D
+//                updates then neither divide by kappa nor hold its divisor, which took four
+//                registers of a core column.
+enum { DIV_IEEE = 0, DIV_EXACT = 1, DIV_RECIP = 2, DIV_EXACT1 = 3 };
 
 template <int FAST, typename T>
 __device__ __forceinline__ T cdiv(T x, const DivC<T>& D) {
@@ -87,6 +97,12 @@ __device__ __forceinline__ T mad(T a, T b, T c) {
 
 __device__ __forceinline__ float qscaled(float x, float d, float r, unsigned lob1, unsigned hib);
 
+template <>
+__device__ __forceinline__ float cdiv<DIV_EXACT, float>(float x, const DivC<float>& D);
+template <>
+__device__ __forceinline__ float cdiv<DIV_EXACT1, float>(float x, const DivC<float>& D) {
+    return cdiv<DIV_EXACT>(x, D);
+}
 template <>
 __device__ __forceinline__ float cdiv<DIV_EXACT, float>(float x, const DivC<float>& D) {
     const unsigned ax = __float_as_uint(x) & 0x7fffffffu;
@@ -116,6 +132,26 @@ __device__ __forceinline__ float qcorr(float x, float d, float r) {
     return copysignf(__fmaf_rn(e, r, q0), x);
 }
 
+// RN(x/d) in double precision for x in the band or zero (see DivC).
+__device__ __forceinline__ double qcorr64(double x, double d, double r) {
+    const double q0 = __dmul_rn(x, r);
+    const double q1 = __fma_rn(__fma_rn(-q0, d, x), r, q0);
+    const double q = __fma_rn(__fma_rn(-q1, d, x), r, q1);
+    return __hiloint2double((__double2hiint(q) & 0x7fffffff) | (__double2hiint(x) & 0x80000000), __double2loint(q));
+}
+
+// The high word of |x| as a band key: 0 for x = 0 only.
+__device__ __forceinline__ unsigned band64(double x) {
+    return (unsigned)(__double2hiint(x) & 0x7fffffff) | (__double2loint(x) != 0 ? 1u : 0u);
+}
+
+template <>
+__device__ __forceinline__ double cdiv<DIV_EXACT, double>(double x, const DivC<double>& D) {
+    const unsigned ax = band64(x);
+    if (ax - 1u >= D.lob - 1u && ax <= D.lob + D.span) return qcorr64(x, D.d, D.r);   // zero wraps into the band
+    return x / D.d;
+}
+
 // q[i] = RN(x[i] / d[i]) for the six derivatives, d = (dy, dz, dx, dz, dx, dy) in the order
 // (x-y, x-z, y-x, y-z, z-x, z-y) of the curl.
 // RN(x/d) for a numerator outside the band.  A normal x below the band is scaled by 2^32
@@ -135,6 +171,26 @@ __device__ __forceinline__ float qscaled(float x, float d, float r, unsigned lob
     return __fdiv_rn(x, d);
 }
 
+// The six derivatives in double precision: one band test for all (lob1, hib: high words).
+__device__ __forceinline__ void div6(const DivC<double>& dx, const DivC<double>& dy, const DivC<double>& dz, unsigned lob1,
+                                     unsigned hib, const double (&x)[6], double (&q)[6]) {
+    const double d[6] = {dy.d, dz.d, dx.d, dz.d, dx.d, dy.d}, r[6] = {dy.r, dz.r, dx.r, dz.r, dx.r, dy.r};
+    unsigned mn = 0xffffffffu, mx = 0u;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        q[i] = qcorr64(x[i], d[i], r[i]);
+        const unsigned ax = band64(x[i]);
+        mn = min(mn, ax - 1u);   // zero wraps to the maximum: excluded from the lower bound
+        mx = max(mx, ax);
+    }
+    if (mn >= lob1 && mx <= hib) return;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const unsigned ax = band64(x[i]);
+        if (ax != 0u && (ax - 1u < lob1 || ax > hib)) q[i] = x[i] / d[i];
+    }
+}
+
 template <int FAST>
 __device__ __forceinline__ void div6(const Div3& D, const float (&x)[6], float (&q)[6]) {
     const float d[6] = {D.dy, D.dz, D.dx, D.dz, D.dx, D.dy};
@@ -142,7 +198,7 @@ __device__ __forceinline__ void div6(const Div3& D, const float (&x)[6], float (
         const float r[6] = {D.ry, D.rz, D.rx, D.rz, D.rx, D.ry};
 #pragma unroll
         for (int i = 0; i < 6; ++i) q[i] = x[i] * r[i];
-    } else if constexpr (FAST == DIV_EXACT) {
+    } else if constexpr (FAST == DIV_EXACT || FAST == DIV_EXACT1) {
         const float r[6] = {D.ry, D.rz, D.rx, D.rz, D.rx, D.ry};
         unsigned mn = 0xffffffffu, mx = 0u;
 #pragma unroll
@@ -170,6 +226,15 @@ __device__ __forceinline__ T sqrt0(T v) {
     return v == T(0) ? T(0) : sqrt(v);
 }
 
+// sqrt(a^2) as the reference rounds it (the square, then its root): that is |a| whenever the
+// square is a normal number (in radix 2 the rounded root of the rounded square is exact).
+template <typename T>
+__device__ __forceinline__ T sqrt_sq(T a) {
+    const T v = a * a;
+    constexpr T lo = sizeof(T) == 4 ? T(FLT_MIN) : T(DBL_MIN), hi = sizeof(T) == 4 ? T(FLT_MAX) : T(DBL_MAX);
+    return v >= lo && v <= hi ? fabs(a) : sqrt0(v);
+}
+
 // The same in a kernel's division mode: the tolerance mode takes v * rsqrt(v) in single
 // precision (the hardware reciprocal square root, a few ulp) instead of the correctly
 // rounded square root's longer sequence.
@@ -195,6 +260,13 @@ struct LayerDev {
     T* psi[4];         // 3-D: x faces Hyx,Hzx,Eyx,Ezx; y: Hxy,Hzy,Exy,Ezy; z: Hxz,Hyz,Exz,Eyz
                        // 2-D: x faces Hyx,Ezx; z faces Hyz,Exz.  1-D: z faces Hyz,Exz.
 };
+
+// A derivative divided by kappa of point q of a layer (DIV_EXACT1: every kappa is 1).
+template <int FAST, typename T>
+__device__ __forceinline__ T over_kappa(const LayerDev<T>& l, int q, T d) {
+    if constexpr (FAST == DIV_EXACT1) return d;
+    else return cdiv<FAST>(d, l.K[q]);
+}
 
 // Material coefficients + pointers to its compact state (materials.jl:335-483).
 template <typename T, typename R>

@@ -87,8 +87,8 @@ __device__ __forceinline__ void cpml_h(const LayerDev<T>& l, int q, int k, T Mh,
     l.psi[3][k] = pb;
     if (S > 0) { h1 = mad<FAST>(Mh, pb, h1); h2 = mad<FAST>(-Mh, pa, h2); }
     else { h1 = mad<FAST>(-Mh, pb, h1); h2 = mad<FAST>(Mh, pa, h2); }
-    da = cdiv<FAST>(da, l.K[q]);
-    db = cdiv<FAST>(db, l.K[q]);
+    da = over_kappa<FAST>(l, q, da);
+    db = over_kappa<FAST>(l, q, db);
 }
 
 // CPML of the H curl in the E update, one face (models.jl:975-1035), psi pair (psi[0],
@@ -102,8 +102,8 @@ __device__ __forceinline__ void cpml_e(const LayerDev<T>& l, int q, int k, T Md2
     l.psi[1][k] = pb;
     if (S > 0) { d1 = mad<FAST>(Md2, pb, d1); d2 = mad<FAST>(-Md2, pa, d2); }
     else { d1 = mad<FAST>(-Md2, pb, d1); d2 = mad<FAST>(Md2, pa, d2); }
-    da = cdiv<FAST>(da, l.K[q]);
-    db = cdiv<FAST>(db, l.K[q]);
+    da = over_kappa<FAST>(l, q, da);
+    db = over_kappa<FAST>(l, q, db);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -565,7 +565,7 @@ __device__ __forceinline__ void h2d_cell(const HParams<T>& p, int accum, long lo
             const T ps = l.B[q] * l.psi[1][k] + l.A[q] * dEzx;
             l.psi[1][k] = ps;
             hy = mad<FAST>(Mh, ps, hy);
-            dEzx = cdiv<FAST>(dEzx, l.K[q]);
+            dEzx = over_kappa<FAST>(l, q, dEzx);
         }
     }
     {
@@ -575,7 +575,7 @@ __device__ __forceinline__ void h2d_cell(const HParams<T>& p, int accum, long lo
             const T ps = l.B[q] * l.psi[1][k] + l.A[q] * dEzx;
             l.psi[1][k] = ps;
             hy = mad<FAST>(Mh, ps, hy);
-            dEzx = cdiv<FAST>(dEzx, l.K[q]);
+            dEzx = over_kappa<FAST>(l, q, dEzx);
         }
     }
     {
@@ -585,7 +585,7 @@ __device__ __forceinline__ void h2d_cell(const HParams<T>& p, int accum, long lo
             const T ps = l.B[q] * l.psi[1][k] + l.A[q] * dExz;
             l.psi[1][k] = ps;
             hy = mad<FAST>(-Mh, ps, hy);
-            dExz = cdiv<FAST>(dExz, l.K[q]);
+            dExz = over_kappa<FAST>(l, q, dExz);
         }
     }
     {
@@ -595,7 +595,7 @@ __device__ __forceinline__ void h2d_cell(const HParams<T>& p, int accum, long lo
             const T ps = l.B[q] * l.psi[1][k] + l.A[q] * dExz;
             l.psi[1][k] = ps;
             hy = mad<FAST>(-Mh, ps, hy);
-            dExz = cdiv<FAST>(dExz, l.K[q]);
+            dExz = over_kappa<FAST>(l, q, dExz);
         }
     }
     hy = mad<FAST>(-Mh, dExz - dEzx, hy);
@@ -641,7 +641,7 @@ __device__ __forceinline__ void e2d_cell(const EParams<T, R>& p, int ix, int iz)
             const T ps = l.B[q] * l.psi[0][k] + l.A[q] * dHyx;
             l.psi[0][k] = ps;
             D2 = mad<FAST>(Md2, ps, D2);
-            dHyx = cdiv<FAST>(dHyx, l.K[q]);
+            dHyx = over_kappa<FAST>(l, q, dHyx);
         }
     }
     {
@@ -651,7 +651,7 @@ __device__ __forceinline__ void e2d_cell(const EParams<T, R>& p, int ix, int iz)
             const T ps = l.B[q] * l.psi[0][k] + l.A[q] * dHyx;
             l.psi[0][k] = ps;
             D2 = mad<FAST>(Md2, ps, D2);
-            dHyx = cdiv<FAST>(dHyx, l.K[q]);
+            dHyx = over_kappa<FAST>(l, q, dHyx);
         }
     }
     {
@@ -661,7 +661,7 @@ __device__ __forceinline__ void e2d_cell(const EParams<T, R>& p, int ix, int iz)
             const T ps = l.B[q] * l.psi[0][k] + l.A[q] * dHyz;
             l.psi[0][k] = ps;
             D0 = mad<FAST>(-Md2, ps, D0);
-            dHyz = cdiv<FAST>(dHyz, l.K[q]);
+            dHyz = over_kappa<FAST>(l, q, dHyz);
         }
     }
     {
@@ -671,7 +671,7 @@ __device__ __forceinline__ void e2d_cell(const EParams<T, R>& p, int ix, int iz)
             const T ps = l.B[q] * l.psi[0][k] + l.A[q] * dHyz;
             l.psi[0][k] = ps;
             D0 = mad<FAST>(-Md2, ps, D0);
-            dHyz = cdiv<FAST>(dHyz, l.K[q]);
+            dHyz = over_kappa<FAST>(l, q, dHyz);
         }
     }
     D0 = Md1 * D0 + Md2 * (T(0) - dHyz);
@@ -727,7 +727,7 @@ __device__ __forceinline__ void h2e_cell(const HParams<T>& p, int accum, long lo
             const T ps = l.B[q] * l.psi[1][k] + l.A[q] * dEyx;
             l.psi[1][k] = ps;
             hz = mad<FAST>(-Mh, ps, hz);
-            dEyx = cdiv<FAST>(dEyx, l.K[q]);
+            dEyx = over_kappa<FAST>(l, q, dEyx);
         }
     }
 #pragma unroll
@@ -738,7 +738,7 @@ __device__ __forceinline__ void h2e_cell(const HParams<T>& p, int accum, long lo
             const T ps = l.B[q] * l.psi[1][k] + l.A[q] * dEyz;
             l.psi[1][k] = ps;
             hx = mad<FAST>(Mh, ps, hx);
-            dEyz = cdiv<FAST>(dEyz, l.K[q]);
+            dEyz = over_kappa<FAST>(l, q, dEyz);
         }
     }
     hx = mad<FAST>(-Mh, T(0) - dEyz, hx);
@@ -786,7 +786,7 @@ __device__ __forceinline__ void e2e_cell(const EParams<T, R>& p, int ix, int iz)
             const T ps = l.B[q] * l.psi[0][k] + l.A[q] * dHzx;
             l.psi[0][k] = ps;
             D1 = mad<FAST>(-Md2, ps, D1);
-            dHzx = cdiv<FAST>(dHzx, l.K[q]);
+            dHzx = over_kappa<FAST>(l, q, dHzx);
         }
     }
 #pragma unroll
@@ -797,7 +797,7 @@ __device__ __forceinline__ void e2e_cell(const EParams<T, R>& p, int ix, int iz)
             const T ps = l.B[q] * l.psi[0][k] + l.A[q] * dHxz;
             l.psi[0][k] = ps;
             D1 = mad<FAST>(Md2, ps, D1);
-            dHxz = cdiv<FAST>(dHxz, l.K[q]);
+            dHxz = over_kappa<FAST>(l, q, dHxz);
         }
     }
     D1 = Md1 * D1 + Md2 * (dHxz - dHzx);
@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(256) h1d_kernel(const __grid_constant__ HParam
     T hy = p.Hy[c];
     if (p.accum) {
         const T a = ex * hy;
-        p.Sa[c] = p.Sa[c] + sqrt0(a * a) * p.dt;
+        p.Sa[c] = p.Sa[c] + sqrt_sq(a) * p.dt;
         if (p.sum_e2) p.E2[c] = p.E2[c] + ex * ex * p.dt;
         guard(p, ex);
     }
@@ -843,7 +843,7 @@ __global__ void __launch_bounds__(256) h1d_kernel(const __grid_constant__ HParam
             const T ps = l.B[q] * l.psi[1][q] + l.A[q] * dExz;
             l.psi[1][q] = ps;
             hy = mad<FAST>(-Mh, ps, hy);
-            dExz = cdiv<FAST>(dExz, l.K[q]);
+            dExz = over_kappa<FAST>(l, q, dExz);
         }
     }
     {
@@ -853,7 +853,7 @@ __global__ void __launch_bounds__(256) h1d_kernel(const __grid_constant__ HParam
             const T ps = l.B[q] * l.psi[1][q] + l.A[q] * dExz;
             l.psi[1][q] = ps;
             hy = mad<FAST>(-Mh, ps, hy);
-            dExz = cdiv<FAST>(dExz, l.K[q]);
+            dExz = over_kappa<FAST>(l, q, dExz);
         }
     }
     hy -= Mh * (T(0) + dExz);
@@ -888,7 +888,7 @@ __global__ void __launch_bounds__(256) e1d_kernel(const __grid_constant__ EParam
             const T ps = l.B[q] * l.psi[0][q] + l.A[q] * dHyz;
             l.psi[0][q] = ps;
             D0 = mad<FAST>(-Md2, ps, D0);
-            dHyz = cdiv<FAST>(dHyz, l.K[q]);
+            dHyz = over_kappa<FAST>(l, q, dHyz);
         }
     }
     {
@@ -898,7 +898,7 @@ __global__ void __launch_bounds__(256) e1d_kernel(const __grid_constant__ EParam
             const T ps = l.B[q] * l.psi[0][q] + l.A[q] * dHyz;
             l.psi[0][q] = ps;
             D0 = mad<FAST>(-Md2, ps, D0);
-            dHyz = cdiv<FAST>(dHyz, l.K[q]);
+            dHyz = over_kappa<FAST>(l, q, dHyz);
         }
     }
     D0 = Md1 * D0 + Md2 * (T(0) - dHyz);
@@ -1004,7 +1004,7 @@ __global__ void __launch_bounds__(256) sums_kernel(const __grid_constant__ HPara
     } else {
         const T hy = p.Hy[c];
         const T a = ex * hy;
-        p.Sa[c] = p.Sa[c] + sqrt0(a * a) * p.dt;
+        p.Sa[c] = p.Sa[c] + sqrt_sq(a) * p.dt;
         if (p.sum_e2) p.E2[c] = p.E2[c] + ex * ex * p.dt;
     }
     guard(p, ex);

@@ -218,8 +218,8 @@ __global__ void __launch_bounds__(AS_TX * AS_TY, LAY ? (FAST == DIV_RECIP ? MFD_
             X.pb[k] = pb;
             hy = mad<FAST>(Mh, pb, hy);
             hz = mad<FAST>(-Mh, pa, hz);
-            dEyx = cdiv<FAST>(dEyx, X.K);
-            dEzx = cdiv<FAST>(dEzx, X.K);
+            dEyx = over_kappa<FAST>(X, dEyx);
+            dEzx = over_kappa<FAST>(X, dEzx);
         }
         if (LAY && yin) {   // cpml_h<-1> of the row's y face
             const float pa = mad<FAST>(Y.B, cya, Y.A * dExy);
@@ -228,8 +228,8 @@ __global__ void __launch_bounds__(AS_TX * AS_TY, LAY ? (FAST == DIV_RECIP ? MFD_
             Y.pb[ky] = pb;
             hx = mad<FAST>(-Mh, pb, hx);
             hz = mad<FAST>(Mh, pa, hz);
-            dExy = cdiv<FAST>(dExy, Y.K);
-            dEzy = cdiv<FAST>(dEzy, Y.K);
+            dExy = over_kappa<FAST>(Y, dExy);
+            dEzy = over_kappa<FAST>(Y, dEzy);
         }
         if (LAY == 2) {   // cpml_h<+1> of the plane's z face
             const int qz = iz - zq0;
@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(AS_TX * AS_TY, LAY ? (FAST == DIV_RECIP ? MFD_
             LZ.psi[3][kz] = pb;
             hx = mad<FAST>(Mh, pb, hx);
             hy = mad<FAST>(-Mh, pa, hy);
-            dExz = cdiv<FAST>(dExz, LZ.K[qz]);
-            dEyz = cdiv<FAST>(dEyz, LZ.K[qz]);
+            dExz = over_kappa<FAST>(LZ, qz, dExz);
+            dEyz = over_kappa<FAST>(LZ, qz, dEyz);
         }
         hx = mad<FAST>(-Mh, dEzy - dEyz, hx);
         hy = mad<FAST>(-Mh, dExz - dEzx, hy);
@@ -451,8 +451,8 @@ __global__ void __launch_bounds__(AS_TX * AS_TY, LAY ? (FAST == DIV_RECIP ? (MAT
             X.pb[k] = pb;
             D1 = mad<FAST>(-Md2, pb, D1);
             D2 = mad<FAST>(Md2, pa, D2);
-            dHyx = cdiv<FAST>(dHyx, X.K);
-            dHzx = cdiv<FAST>(dHzx, X.K);
+            dHyx = over_kappa<FAST>(X, dHyx);
+            dHzx = over_kappa<FAST>(X, dHzx);
         }
         if (LAY && yin) {   // cpml_e<+1> of the row's y face
             const float pa = mad<FAST>(Y.B, cya, Y.A * dHxy);
@@ -461,8 +461,8 @@ __global__ void __launch_bounds__(AS_TX * AS_TY, LAY ? (FAST == DIV_RECIP ? (MAT
             Y.pb[ky] = pb;
             D0 = mad<FAST>(Md2, pb, D0);
             D2 = mad<FAST>(-Md2, pa, D2);
-            dHxy = cdiv<FAST>(dHxy, Y.K);
-            dHzy = cdiv<FAST>(dHzy, Y.K);
+            dHxy = over_kappa<FAST>(Y, dHxy);
+            dHzy = over_kappa<FAST>(Y, dHzy);
         }
         if (LAY == 2) {   // cpml_e<-1> of the plane's z face
             const int qz = iz - zq0;
@@ -473,8 +473,8 @@ __global__ void __launch_bounds__(AS_TX * AS_TY, LAY ? (FAST == DIV_RECIP ? (MAT
             LZ.psi[1][kz] = pb;
             D0 = mad<FAST>(-Md2, pb, D0);
             D1 = mad<FAST>(Md2, pa, D1);
-            dHxz = cdiv<FAST>(dHxz, LZ.K[qz]);
-            dHyz = cdiv<FAST>(dHyz, LZ.K[qz]);
+            dHxz = over_kappa<FAST>(LZ, qz, dHxz);
+            dHyz = over_kappa<FAST>(LZ, qz, dHyz);
         }
         D0 = mad<FAST>(Md1, D0, Md2 * (dHzy - dHyz));
         D1 = mad<FAST>(Md1, D1, Md2 * (dHxz - dHzx));

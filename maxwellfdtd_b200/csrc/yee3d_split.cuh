@@ -54,12 +54,14 @@ __device__ __forceinline__ void slab_row(const SplitBox& s, int ny, int r, int& 
 }
 
 // The six curl derivatives of a cell, q = num / (dy, dz, dx, dz, dx, dy): for single precision
-// the verified branch-free division (div6), for double precision IEEE division.
+// the verified branch-free division (div6), for double precision its own or IEEE division.
 template <typename T, int FAST>
 __device__ __forceinline__ void curl_div(const Div3& D3, const DivC<T>& ddx, const DivC<T>& ddy, const DivC<T>& ddz,
                                          const T (&num)[6], T (&q)[6]) {
     if constexpr (sizeof(T) == 4) {
         div6<FAST>(D3, num, q);
+    } else if constexpr (FAST == DIV_EXACT) {
+        div6(ddx, ddy, ddz, D3.lob1, D3.hib, num, q);
     } else {
         q[0] = cdiv<FAST>(num[0], ddy); q[1] = cdiv<FAST>(num[1], ddz); q[2] = cdiv<FAST>(num[2], ddx);
         q[3] = cdiv<FAST>(num[3], ddz); q[4] = cdiv<FAST>(num[4], ddx); q[5] = cdiv<FAST>(num[5], ddy);
@@ -103,6 +105,13 @@ __device__ __forceinline__ XCol<T> xcol(const LayerDev<T>& lxl, const LayerDev<T
         x.K = DivC<T>{};
     }
     return x;
+}
+
+// A derivative over the column's kappa (DIV_EXACT1: every kappa of the model is 1).
+template <int FAST, typename T>
+__device__ __forceinline__ T over_kappa(const XCol<T>& x, T d) {
+    if constexpr (FAST == DIV_EXACT1) return d;
+    else return cdiv<FAST>(d, x.K);
 }
 
 template <typename T>
@@ -192,8 +201,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? MFD_CORE_MINB : 2) h3d_c
             X.pb[k] = pb;
             hy = mad<FAST>(Mh, pb, hy);
             hz = mad<FAST>(-Mh, pa, hz);
-            dEyx = cdiv<FAST>(dEyx, X.K);
-            dEzx = cdiv<FAST>(dEzx, X.K);
+            dEyx = over_kappa<FAST>(X, dEyx);
+            dEzx = over_kappa<FAST>(X, dEzx);
         }
         hx = mad<FAST>(-Mh, dEzy - dEyz, hx);
         hy = mad<FAST>(-Mh, dExz - dEzx, hy);
@@ -370,8 +379,8 @@ __global__ void __launch_bounds__(256, RESP ? 2 : (sizeof(T) == 4 ? MFD_CORE_MIN
             X.pb[k] = pb;
             D1 = mad<FAST>(-Md2, pb, D1);
             D2 = mad<FAST>(Md2, pa, D2);
-            dHyx = cdiv<FAST>(dHyx, X.K);
-            dHzx = cdiv<FAST>(dHzx, X.K);
+            dHyx = over_kappa<FAST>(X, dHyx);
+            dHzx = over_kappa<FAST>(X, dHzx);
         }
         D0 = mad<FAST>(Md1, D0, Md2 * (dHzy - dHyz));
         D1 = mad<FAST>(Md1, D1, Md2 * (dHxz - dHzx));
