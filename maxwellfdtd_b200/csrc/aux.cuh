@@ -156,14 +156,11 @@ struct MonParams {
     const MonDev<T>* mons;
 };
 
-// Grid row blockIdx.y = monitor; a thread gathers every component of one point (one cell
-// index load, the component loads independent of each other).
+// Point j (padded cell `cell`) of a monitor: every component of one point, the component loads
+// independent of each other.
 template <typename T>
-__global__ void __launch_bounds__(256) monitor_gather_kernel(const __grid_constant__ MonParams<T> p, long long it0, int slot) {
-    const MonDev<T>& M = p.mons[blockIdx.y];
-    const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (j >= M.npts) return;
-    const int cell = M.cells[j];
+__device__ __forceinline__ void monitor_store(const MonParams<T>& p, const MonDev<T>& M, long long j, int cell, long long it0,
+                                              int slot) {
     T v[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k)
@@ -175,6 +172,18 @@ __global__ void __launch_bounds__(256) monitor_gather_kernel(const __grid_consta
         if (hist) M.hist[((long long)k * p.nt + it0) * M.npts + j] = v[k];
         else M.ring[((long long)slot * p.ncomp + k) * M.npts + j] = v[k];
     }
+}
+
+template <typename T>
+__device__ __forceinline__ void monitor_point(const MonParams<T>& p, int m, long long j, long long it0, int slot) {
+    const MonDev<T>& M = p.mons[m];
+    if (j < M.npts) monitor_store(p, M, j, M.cells[j], it0, slot);
+}
+
+// Grid row blockIdx.y = monitor.
+template <typename T>
+__global__ void __launch_bounds__(256) monitor_gather_kernel(const __grid_constant__ MonParams<T> p, long long it0, int slot) {
+    monitor_point(p, blockIdx.y, blockIdx.x * (long long)blockDim.x + threadIdx.x, it0, slot);
 }
 
 // Summed field monitor: hist[k][it] = sum over points (block reduction in T).

@@ -31,6 +31,7 @@
 #include "yee3d_async.cuh"
 #include "yee3d_split.cuh"
 #include "batch.cuh"
+#include "resident.cuh"
 #include "geometry.cuh"
 
 namespace mfd {
@@ -443,6 +444,13 @@ class Engine : public HandleBase {
     bool resp_fused = false;   // material response inside the E kernel of the core rows (RESP)
     int kcount = 1;             // kernels issued by the current launch() call
 
+    // Small models: many steps in one cooperative launch (resident.cuh)
+    bool resident = false;
+    ResidentParams<T> res_p{};
+    int res_blocks = 0, res_threads = 0, res_smem = 0;
+    int* d_resfault = nullptr;
+    int h_resfault = 0;
+
     // timing
     bool profiling = false;
     double k_ms[KC_N] = {};
@@ -773,8 +781,207 @@ class Engine : public HandleBase {
         h_flags = h_flags_v.data();
         MFD_CK(cudaStreamSynchronize(st));
         init_split();
-        mon_apart = overlap && monitors_apart_from_sources(d);
+        init_resident(d);
+        mon_apart = overlap && !resident && monitors_apart_from_sources(d);
         if (mon_apart) make_side_stream();
+    }
+
+    // ---- resident steps (resident.cuh) -------------------------------------------------
+    // Cells up to which the resident steps are the faster way (us per step, separate launches
+    // against resident, dispersive model with CPML, one point source and four monitors):
+    //   1-D, any: 3 000 cells 24.3 / 4.5, 60 000 35.0 / 5.0;
+    //   2-D float 301 x 300 22.8 / 6.8, 701 x 700 27.7 / 18.0, 1101 x 1100 36.9 / 34.0;
+    //   2-D double 301 x 300 24.6 / 9.7, 901 x 900 35.9 / 31.7, 1101 x 1100 48.4 / 49.2;
+    //   3-D float 46 x 45 x 44 36.7 / 9.0, 91 x 90 x 89 54.0 / 43.3 (tolerance mode 83.5 / 36.5);
+    //   3-D double 46 x 45 x 44 37.5 / 12.7, 91 x 90 x 89 69.8 / 57.4, 100^3 82 / 102.
+    static long long resident_limit(int nd) { return nd == 3 ? 750000 : 1000000; }
+
+    template <typename F_>
+    void with_resident_kernel(F_&& f) {
+        if constexpr (std::is_same<R, double>::value) {
+            auto pick = [&](auto fs, auto dm) {
+                constexpr int FS = decltype(fs)::value, D = decltype(dm)::value;
+                if (any_geom) f(resident_kernel<T, R, FS, true, D>);
+                else f(resident_kernel<T, R, FS, false, D>);
+            };
+            auto dims = [&](auto dm) {
+                if (ndim == 1) pick(std::integral_constant<int, 1>{}, dm);
+                else if (ndim == 3) pick(std::integral_constant<int, 3>{}, dm);
+                else if (ey2) pick(std::integral_constant<int, FSET_EY2>{}, dm);
+                else pick(std::integral_constant<int, 2>{}, dm);
+            };
+            if (recip) dims(std::integral_constant<int, DIV_RECIP>{});
+            else dims(std::integral_constant<int, DIV_EXACT>{});
+        }
+    }
+
+    // Which models step by the resident kernel, and its per-block lists of source and monitor
+    // points.  Not: models of a server (overlap = false: many run at once, and a cooperative
+    // launch waits until all of its blocks fit), TFSF recording, plasma (its transcendental
+    // code, and compute-bound), more than three poles, divisors that failed the check, CPML layers that overlap, more than RES_MAXOPS sources.
+    void init_resident(const mfd_desc* d) {
+        if (!std::is_same<R, double>::value || !overlap || record || any_plasma || N > resident_limit(ndim)) return;
+        if (!recip && !fastdiv) return;
+        // an explicit choice of the 3-D kernels keeps them
+        if (ndim == 3 && (std::getenv("MFD_KERNEL3D") || std::getenv("MFD_CORE_ASYNC"))) return;
+        for (int g : response_mats)
+            if (mats_host[g - 1].nq > 3) return;
+        for (int f = 0; f < 6; f += 2)   // a cell in both layers of an axis (they overlap)
+            if (lay[f].nb && lay[f + 1].nb && lay[f].ib > lay[f + 1].ib - 1) return;
+        const int nops = (int)srcs.size() + (tfsf ? 1 : 0);
+        if (nops > RES_MAXOPS) return;
+        int per_sm = 0, sms = 0, coop = 0;
+        with_resident_kernel([&](auto k) { MFD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, RES_THREADS<T>, 0)); });
+        MFD_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        MFD_CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        if (per_sm < 1 || !coop) return;
+        ResidentParams<T>& p = res_p;
+        p.ncell = (int)N;
+        res_blocks = (int)std::min<long long>((long long)per_sm * sms, (N + RES_MINCELLS - 1) / RES_MINCELLS);
+        p.per = (int)((N + res_blocks - 1) / res_blocks);
+        res_blocks = (int)((N + p.per - 1) / p.per);
+        // every round of the block's threads over its cells equally full
+        const int rounds = (p.per + RES_THREADS<T> - 1) / RES_THREADS<T>;
+        res_threads = (int)round_up((p.per + rounds - 1) / rounds, 32);
+        // shared-memory tables, as far as they fit beside the static ones in 46 KB per block
+        // (two blocks of an SM then leave most of it to L1)
+        res_smem = 0;
+        auto place = [&](long long bytes) {
+            if (bytes <= 0 || res_smem + bytes > 46 * 1024) return -1;
+            const int o = res_smem;
+            res_smem += (int)round_up(bytes, 16);
+            return o;
+        };
+        p.nmat = nmat;
+        p.k1 = kappa_one;
+        p.o_geom = p.o_mats = p.o_math = p.o_rect = -1;
+        for (int f = 0; f < 6; ++f)
+            p.o_lay[f] = place((long long)lay[f].nb * (long long)(sizeof(DivC<T>) + 2 * sizeof(T)));
+        p.o_ops = place((long long)nops * (long long)sizeof(ResOp<T>));
+        p.o_mon = place((long long)mon_p.nmon * (long long)sizeof(MonDev<T>));
+        if (any_geom) {
+            p.o_mats = place((long long)nmat * (long long)sizeof(MatDev<T, R>));
+            if (p.o_mats >= 0) {
+                p.o_math = place((long long)nmat * (long long)sizeof(T));
+                if (p.o_math < 0) p.o_mats = -1;
+            }
+            long long w = 0;   // widest run of padded cells of a block
+            for (int b = 0; b < res_blocks; ++b) {
+                const long long l0 = (long long)b * p.per, l1 = std::min(l0 + p.per, N) - 1;
+                w = std::max(w, pad_index(l1) - pad_index(l0) + 1);
+            }
+            p.o_geom = place(w);
+        }
+        if (tfsf) p.o_rect = place((long long)sizeof(RectParams<T>));
+        // lists by block: point indices of each point source, (statement, local) pairs of the
+        // TFSF replay, (monitor, point) pairs
+        std::vector<int> all;
+        std::vector<std::pair<size_t, size_t>> at;   // (offsets, entries) of each list within `all`
+        auto add_list = [&](int width, auto&& each) {   // each(emit): emit(cell, a, b) for every entry
+            std::vector<int> off(res_blocks + 1, 0);
+            each([&](long long cell, int, int) { off[cell / p.per + 1]++; });
+            for (int b = 0; b < res_blocks; ++b) off[b + 1] += off[b];
+            std::vector<int> pos(off.begin(), off.end() - 1), ent((size_t)off[res_blocks] * width);
+            each([&](long long cell, int a, int b) {
+                const int k = pos[cell / p.per]++;
+                ent[(size_t)k * width] = a;
+                if (width == 2) ent[(size_t)k * 2 + 1] = b;
+            });
+            at.push_back({all.size(), all.size() + off.size()});
+            all.insert(all.end(), off.begin(), off.end());
+            all.insert(all.end(), ent.begin(), ent.end());
+        };
+        std::vector<ResOp<T>> ops;
+        for (size_t i = 0; i <= srcs.size(); ++i) {
+            if (tfsf && (int)i == tfsf_order) {
+                add_list(2, [&](auto&& emit) {
+                    for (int k = 0; k < tfsf_p.n; ++k) {
+                        const RectStmt& q = tfsf_p.s[k];
+                        int local = 0;
+                        for (int z = q.z0; z <= q.z1; ++z)
+                            for (int y = q.y0; y <= q.y1; ++y)
+                                for (int x = q.x0; x <= q.x1; ++x, ++local) emit((long long)x + (long long)nx * (y + (long long)ny * z), k, local);
+                    }
+                });
+                ResOp<T> o{};
+                o.tfsf = 1;
+                ops.push_back(o);
+            }
+            if (i < srcs.size()) {
+                const int64_t* cells = d->srcs[i].cells;
+                const Src& S = srcs[i];
+                add_list(1, [&](auto&& emit) { for (long long j = 0; j < S.npts; ++j) emit(cells[j], (int)j, 0); });
+                ResOp<T> o{};
+                o.kind = S.kind; o.coeff = S.coeff; o.F = F[S.comp]; o.cells = S.cells; o.wave = S.wave; o.amp = S.amp;
+                o.gt = S.gt; o.npts = S.npts;
+                ops.push_back(o);
+            }
+        }
+        p.nops = (int)ops.size();
+        p.nmon = mon_p.nmon;
+        if (p.nmon)
+            add_list(2, [&](auto&& emit) {
+                for (int m = 0; m < d->nmon; ++m)
+                    for (long long j = 0; j < d->mons[m].npts; ++j) emit(d->mons[m].cells[j], m, (int)j);
+            });
+        int most = 0;   // points of one block
+        for (int b = 0; b < res_blocks; ++b) {
+            int n = 0;
+            for (auto& l : at) n += all[l.first + b + 1] - all[l.first + b];
+            most = std::max(most, n);
+        }
+        p.o_pts = place((long long)most * (long long)sizeof(ResPoint));
+        p.npts_cap = p.o_pts < 0 ? 0 : most;
+        if (p.o_pts < 0) p.o_pts = 0;
+        {   // the grid must still be resident at once with that much shared memory
+            int fit = 0;
+            with_resident_kernel([&](auto k) { MFD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, RES_THREADS<T>, (size_t)res_smem)); });
+            if ((long long)fit * sms < res_blocks) return;
+        }
+        if (!all.empty()) {
+            const int* da = upload(all.data(), all.size());
+            for (size_t o = 0; o < ops.size(); ++o) { ops[o].off = da + at[o].first; ops[o].list = da + at[o].second; }
+            if (p.nmon) { p.moff = da + at.back().first; p.mlist = da + at.back().second; }
+        }
+        if (!ops.empty()) p.ops = upload(ops.data(), ops.size());
+        if (tfsf) p.rp = upload(&tfsf_p, 1);
+        p.mp = mon_p;
+        p.dt = dt;
+        p.bar = dalloc<unsigned>(1, false);
+        p.fault = d_resfault = dalloc<int>(1, false);
+        MFD_CK(cudaStreamSynchronize(st));
+        resident = true;
+    }
+
+    // Steps it .. it + n - 1 in one launch.
+    void launch_resident(int64_t it, int n, int accum) {
+        HParams<T> hp = hparams(accum, it - 1);
+        EParams<T, R> ep = eparams();
+        int slot0 = 0;
+        if (!mons_host.empty() && need_ring) {
+            if (ring_used == 0) ring_first = it - 1;
+            slot0 = ring_used;
+        }
+        MFD_CK(cudaMemsetAsync(res_p.bar, 0, sizeof(unsigned), st));
+        launch(KC_H, [&] {
+            with_resident_kernel([&](auto k) {
+                long long first = it;
+                void* args[] = {&hp, &ep, &d3, &res_p, &first, &n, &accum, &slot0};
+                MFD_CK(cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)res_blocks), dim3((unsigned)res_threads), args, (size_t)res_smem, st));
+            });
+        });
+        if (!mons_host.empty() && need_ring) ring_used += n;
+    }
+    // How many steps from `it` one launch may take: up to b, to the next snapshot, to the end of
+    // the monitors' staging ring, and a bound on one kernel's length.
+    int resident_steps(int64_t it, int64_t b) const {
+        int64_t n = std::min<int64_t>(b - it + 1, 4096);
+        if (snap_next < snap_steps.size()) n = std::min<int64_t>(n, snap_steps[snap_next] - it + 1);
+        if (!mons_host.empty() && need_ring) n = std::min<int64_t>(n, ring_k - ring_used);
+        return (int)n;
+    }
+    void check_resident() const {
+        if (h_resfault) throw Error(MFD_ERR_TIMEOUT, "a grid barrier of the resident steps did not complete within its wait limit");
     }
 
     void make_side_stream() {
@@ -1745,6 +1952,15 @@ class Engine : public HandleBase {
         MFD_CK(cudaSetDevice(dev));
         MFD_CK(cudaEventRecord(run_ev[0], st));
         for (int64_t it = a; it <= b; ++it) {
+            if (resident && !profiling) {
+                const int n = resident_steps(it, b);
+                launch_resident(it, n, (it > a || sums_pending) ? 1 : 0);
+                sums_pending = false;
+                it += n - 1;
+                fold_if_full();
+                if (snap_next < snap_steps.size() && snap_steps[snap_next] == it) snapshot();
+                continue;
+            }
             launch_H((it > a || sums_pending) ? 1 : 0, it - 1);
             sums_pending = false;
             launch_E((int)((it - 1) & 1));
@@ -1836,8 +2052,10 @@ class Engine : public HandleBase {
         MFD_CK(cudaMemcpyAsync(h_flags + (a - 1), d_flags + (a - 1), (size_t)(b - a + 1) * sizeof(int),
                                cudaMemcpyDeviceToHost, st));
         if (tc_fold) MFD_CK(cudaMemcpyAsync(&h_tcfault, d_tcfault, sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (resident) MFD_CK(cudaMemcpyAsync(&h_resfault, d_resfault, sizeof(int), cudaMemcpyDeviceToHost, st));
         bounded_sync(st);
         check_fold();
+        check_resident();
         float ms = 0;
         MFD_CK(cudaEventElapsedTime(&ms, run_ev[0], run_ev[1]));
         run_ms = ms;

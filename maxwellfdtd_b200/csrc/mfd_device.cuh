@@ -431,12 +431,13 @@ __device__ __forceinline__ void material_cell(const MatDev<T, R>* __restrict__ m
 // material_cell with the number of poles NQ known at compile time: every load of the cell
 // (E^n, both polarisation buffers of every pole, the plasma state) is issued before any
 // store, so the poles do not become dependent round trips to memory.  The arithmetic is
-// material_cell's, expression for expression.  bi is the cell's index in the material's box.
-template <typename T, typename R, int NC, int NQ>
+// material_cell's, expression for expression.  bi is the cell's index in the material's box.  PLASMA = false
+// leaves the plasma code out, for callers whose models hold no plasma.
+template <typename T, typename R, int NC, int NQ, bool PLASMA = true>
 __device__ __forceinline__ void material_cell_n(const MatDev<T, R>* __restrict__ m, long long bi,
                                                 T* const* E, long long c, const T* Dv, int cur, T dt) {
     const T Me = m->Me;
-    const bool plasma = m->plasma != 0;
+    const bool plasma = PLASMA && m->plasma != 0;
     const long long bs = m->bsize;
     T sumP[NC];
 #pragma unroll
