@@ -353,6 +353,17 @@ __global__ void __launch_bounds__(256) scatter_state_kernel(const MatDev<T, R>* 
     else ((double*)out)[c] = pl ? 0.0 + (double)(m->rho[bi] * m->rho0) : 0.0;
 }
 
+// Rows row0 .. of a padded array (nx of px elements each) written densely, n elements from
+// dense[0] on: what a read-back copies out when rows are short.
+template <typename U>
+__global__ void __launch_bounds__(256) pack_rows_kernel(const U* __restrict__ src, U* __restrict__ dense, int nx, int px,
+                                                        long long row0, long long n) {
+    for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < n; o += (long long)gridDim.x * blockDim.x) {
+        const long long row = o / nx;
+        dense[o] = src[(row0 + row) * px + (o - row * nx)];
+    }
+}
+
 // The same values for the z-planes z0 .. z0 + gridDim.z - 1 only, written densely (x fastest,
 // then y, then z) from `out`, for the allocation-free read that stages a few planes at a time
 // through a fixed device buffer.

@@ -97,14 +97,14 @@ static double wait_timeout_s() {
 static void bounded_sync(cudaStream_t st) {
     auto t0 = std::chrono::steady_clock::now();
     const double limit = wait_timeout_s();
-    int spins = 0;
     while (true) {
         cudaError_t e = cudaStreamQuery(st);
         if (e == cudaSuccess) return;
         if (e != cudaErrorNotReady) throw Error(MFD_ERR_CUDA, std::string("stream: ") + cudaGetErrorString(e));
-        double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (el > limit) throw Error(MFD_ERR_TIMEOUT, "device work did not finish within the wait limit");
-        if (++spins > 64) std::this_thread::sleep_for(std::chrono::microseconds(spins > 1000 ? 200 : 20));
+        // short waits (a read-back, a few steps) are polled; longer ones sleep, at first briefly
+        if (el > 300e-6) std::this_thread::sleep_for(std::chrono::microseconds(el > 50e-3 ? 200 : 20));
     }
 }
 
@@ -488,34 +488,70 @@ class Engine : public HandleBase {
     // order: the model state that mfd_read_state / mfd_write_state carry.
     std::vector<std::pair<void*, size_t>> state_bufs;
 
+    // A model has some 70 device arrays, most of them small, and with many models alive each
+    // cudaMallocAsync cost 25 us and more (32 2-D models: 3.5 ms of mfd_create each, 0.5 now).  Arrays
+    // up to ARENA_MAX are cut from chunks that grow with the model; larger ones have their own.
+    static constexpr size_t ARENA_MAX = 4u << 20;
+    char* chunk = nullptr;
+    size_t chunk_left = 0, chunk_next = 256u << 10;
+
+    void* raw_alloc(size_t n) {
+        void* p = nullptr;
+        cudaError_t e = cudaMallocAsync(&p, n, st);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            throw Error(MFD_ERR_OOM, "device allocation of " + std::to_string(n) + " bytes failed: " + cudaGetErrorString(e));
+        }
+        allocs.push_back(p);
+        MFD_CK(cudaMemsetAsync(p, 0, n, st));
+        return p;
+    }
+
     template <typename U>
     U* dalloc(size_t n, bool state = true) {
         if (n == 0) n = 1;
-        void* p = nullptr;
-        cudaError_t e = cudaMallocAsync(&p, n * sizeof(U), st);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            throw Error(MFD_ERR_OOM, "device allocation of " + std::to_string(n * sizeof(U)) + " bytes failed: " + cudaGetErrorString(e));
+        const size_t b = n * sizeof(U), room = (size_t)round_up((long long)b, 256);
+        void* p;
+        if (b > ARENA_MAX) {
+            p = raw_alloc(b);
+        } else {
+            if (room > chunk_left) {
+                chunk_left = std::max(room, chunk_next);
+                chunk_next = std::min(2 * chunk_next, 2 * ARENA_MAX);
+                chunk = (char*)raw_alloc(chunk_left);
+            }
+            p = chunk;
+            chunk += room;
+            chunk_left -= room;
         }
-        allocs.push_back(p);
-        bytes += (int64_t)(n * sizeof(U));
-        MFD_CK(cudaMemsetAsync(p, 0, n * sizeof(U), st));
-        if (state) state_bufs.push_back({p, n * sizeof(U)});
+        bytes += (int64_t)b;
+        if (state) state_bufs.push_back({p, b});
         return (U*)p;
+    }
+
+    // Copies host data that stays where it is until init's last synchronisation: the
+    // descriptor's arrays, members of this object, and vectors handed over (upload_own).  One
+    // synchronisation per model instead of one per array.
+    std::vector<std::shared_ptr<void>> held;
+
+    template <typename U>
+    U* upload_own(std::vector<U>&& v) {
+        auto h = std::make_shared<std::vector<U>>(std::move(v));
+        held.push_back(h);
+        return upload(h->data(), h->size());
     }
 
     template <typename U>
     U* upload(const U* h, size_t n) {
         U* d = dalloc<U>(n, false);
         if (n) MFD_CK(cudaMemcpyAsync(d, h, n * sizeof(U), cudaMemcpyHostToDevice, st));
-        MFD_CK(cudaStreamSynchronize(st));   // the host buffer may be a temporary
         return d;
     }
 
     template <typename U>
     U* upload_cast(const double* h, size_t n) {
         std::vector<U> tmp(h, h + n);
-        return upload(tmp.data(), n);
+        return upload_own(std::move(tmp));
     }
 
     long long pad_index(long long c) const {   // dense x-fastest -> padded
@@ -718,7 +754,7 @@ class Engine : public HandleBase {
             }
         }
         if (nmat) {
-            matMh = upload(mh.data(), nmat);
+            matMh = upload_own(std::move(mh));
             mats_dev = upload(mats_host.data(), nmat);
         }
         // CPML
@@ -741,7 +777,7 @@ class Engine : public HandleBase {
                     fastdiv = fastdiv && D.ok;
                     if (D.d != T(1)) kappa_one = false;
                 }
-                lay[f].K = upload(kv.data(), kv.size());
+                lay[f].K = upload_own(std::move(kv));
             }
             lay[f].A = upload_cast<T>(L.A, L.nb);
             lay[f].B = upload_cast<T>(L.B, L.nb);
@@ -764,7 +800,7 @@ class Engine : public HandleBase {
                 if (s.cells[j] < 0 || s.cells[j] >= N) throw Error(MFD_ERR_INVALID, "source cell out of range");
                 cells[j] = pad_index(s.cells[j]);
             }
-            S.cells = upload(cells.data(), cells.size());
+            S.cells = upload_own(std::move(cells));
             if (s.wave) S.wave = upload(s.wave, (size_t)nt * s.npts);
             else {
                 if (!s.amp || !s.gt) throw Error(MFD_ERR_INVALID, "source needs wave or amp+gt");
@@ -779,11 +815,11 @@ class Engine : public HandleBase {
         d_flags = dalloc<int>((size_t)nt);
         h_flags_v.assign((size_t)nt, 0);
         h_flags = h_flags_v.data();
-        MFD_CK(cudaStreamSynchronize(st));
         init_split();
         init_resident(d);
         mon_apart = overlap && !resident && monitors_apart_from_sources(d);
-        if (mon_apart) make_side_stream();
+        MFD_CK(cudaStreamSynchronize(st));
+        held.clear();
     }
 
     // ---- resident steps (resident.cuh) -------------------------------------------------
@@ -939,17 +975,16 @@ class Engine : public HandleBase {
             if ((long long)fit * sms < res_blocks) return;
         }
         if (!all.empty()) {
-            const int* da = upload(all.data(), all.size());
+            const int* da = upload_own(std::move(all));
             for (size_t o = 0; o < ops.size(); ++o) { ops[o].off = da + at[o].first; ops[o].list = da + at[o].second; }
             if (p.nmon) { p.moff = da + at.back().first; p.mlist = da + at.back().second; }
         }
-        if (!ops.empty()) p.ops = upload(ops.data(), ops.size());
+        if (!ops.empty()) p.ops = upload_own(std::move(ops));
         if (tfsf) p.rp = upload(&tfsf_p, 1);
         p.mp = mon_p;
         p.dt = dt;
         p.bar = dalloc<unsigned>(1, false);
         p.fault = d_resfault = dalloc<int>(1, false);
-        MFD_CK(cudaStreamSynchronize(st));
         resident = true;
     }
 
@@ -1027,7 +1062,6 @@ class Engine : public HandleBase {
         sbox = SplitBox{yl, yr, zl, zr, zc3, (zl + nz - zr) * ny};
         slab_rows = (long long)sbox.nzr + (long long)(zr - zl) * (yl + ny - yr);
         use_split = true;
-        if (overlap) make_side_stream();
         // rows and planes of the core box that hold material cells, widened to the staged
         // E kernel's tiles (AS_TY rows, async_zc planes from the core box's corner)
         // The material response runs inside the core-row E kernel that covers the materials'
@@ -1223,7 +1257,6 @@ class Engine : public HandleBase {
         for (int k = 0; k < narr; ++k)
             if (nonzero[k]) p.arr[k] = upload((const T*)d->tfsf.inc[k], (size_t)clen[k] * nt);
         tfsf = n > 0;
-        MFD_CK(cudaStreamSynchronize(st));
     }
 
     // Record statements: sources.jl:372-384, 534-550, 839-877.
@@ -1351,7 +1384,7 @@ class Engine : public HandleBase {
                 if (a.cells[j] < 0 || a.cells[j] >= N) throw Error(MFD_ERR_INVALID, "monitor cell out of range");
                 cells[j] = (int)pad_index(a.cells[j]);
             }
-            M.cells = upload(cells.data(), cells.size());
+            M.cells = upload_own(std::move(cells));
             if (a.kind == MFD_MON_FIELD) {
                 if (M.sum) M.hist = dalloc<T>((size_t)ncomp_mon * nt);
                 else M.hist = dalloc<T>((size_t)ncomp_mon * nt * a.npts);
@@ -1387,7 +1420,6 @@ class Engine : public HandleBase {
         mon_p.nt = nt;
         for (int k = 0; k < ncomp_mon; ++k) mon_p.comp[k] = F[mon_comps[k]];
         mon_p.mons = mons_dev;
-        MFD_CK(cudaStreamSynchronize(st));
     }
 
     // ---------------------------------------------------------------------------------
@@ -1950,6 +1982,9 @@ class Engine : public HandleBase {
         if (a != done + 1 || b < a - 1 || b > nt) { err = "steps must be consecutive and within 1..Nt"; return MFD_ERR_INVALID; }
         if (b < a) return MFD_OK;
         MFD_CK(cudaSetDevice(dev));
+        // the side streams of the split updates and of the gather, at the first steps that use
+        // them (a model stepped by a batch or by the resident kernel never does)
+        if (overlap && (use_split || mon_apart) && (!resident || profiling)) make_side_stream();
         MFD_CK(cudaEventRecord(run_ev[0], st));
         for (int64_t it = a; it <= b; ++it) {
             if (resident && !profiling) {
@@ -2075,8 +2110,42 @@ class Engine : public HandleBase {
         return MFD_OK;
     }
 
-    void copy_out(const void* dsrc, void* hdst, size_t esize) {
+    // A padded array to a dense host buffer.  The copy engine moves a pitched copy row by row:
+    // rows of 244 bytes (nx = 61) came at 5.8 GB/s and rows of 200-500 bytes at 16 GB/s, where
+    // rows of 924 bytes reach 44.  Shorter rows are therefore packed on the device (a few us)
+    // and copied densely, PACK_BYTES at a time (61 x 48 x 55: 11 arrays and 24 traces 1.28 -> 0.67 ms;
+    // 32 models of 48-128 cells a side: 41 -> 34 ms).  noalloc: the
+    // caller's read may not take device memory.
+    static constexpr size_t PACK_ROW = 1024, PACK_BYTES = 8u << 20;
+    unsigned char* pack_buf = nullptr;
+
+    template <typename U>
+    void copy_packed(const void* dsrc, void* hdst) {
+        const size_t cap = std::min((size_t)N * sizeof(double), PACK_BYTES);   // holds a row of any element type
+        const long long rows = (long long)ny * nz, per = (long long)(cap / sizeof(U)) / nx;
+        if (!pack_buf) pack_buf = dalloc<unsigned char>(cap, false);
+        for (long long r = 0; r < rows; r += per) {
+            const long long n = std::min(per, rows - r) * nx;
+            pack_rows_kernel<U><<<(unsigned)std::min((n + 255) / 256, 148ll * 8), 256, 0, st>>>((const U*)dsrc, (U*)pack_buf, nx, px, r, n);
+            MFD_CK(cudaGetLastError());
+            MFD_CK(cudaMemcpyAsync((U*)hdst + r * nx, pack_buf, (size_t)n * sizeof(U), cudaMemcpyDeviceToHost, st));
+        }
+    }
+
+    void copy_out(const void* dsrc, void* hdst, size_t esize, bool noalloc = false) {
         MFD_CK(cudaSetDevice(dev));
+        if (nx == px) {
+            MFD_CK(cudaMemcpyAsync(hdst, dsrc, (size_t)N * esize, cudaMemcpyDeviceToHost, st));
+            bounded_sync(st);
+            return;
+        }
+        if (!noalloc && (size_t)nx * esize < PACK_ROW) {
+            if (esize == 1) copy_packed<uint8_t>(dsrc, hdst);
+            else if (esize == 4) copy_packed<uint32_t>(dsrc, hdst);
+            else copy_packed<uint64_t>(dsrc, hdst);
+            bounded_sync(st);
+            return;
+        }
         MFD_CK(cudaMemcpy2DAsync(hdst, (size_t)nx * esize, dsrc, (size_t)px * esize, (size_t)nx * esize, (size_t)ny * nz,
                                  cudaMemcpyDeviceToHost, st));
         bounded_sync(st);
@@ -2138,7 +2207,12 @@ class Engine : public HandleBase {
     bool noalloc_ready = false;
     int read_integral_noalloc(int which, void* dst) override {
         MFD_CK(cudaSetDevice(dev));
-        if (which == MFD_INT_SA || which == MFD_INT_E2) return read_integral(which, dst);
+        if (which == MFD_INT_SA || (which == MFD_INT_E2 && E2)) {
+            settle();
+            copy_out(which == MFD_INT_SA ? Sa : E2, dst, sizeof(T), true);
+            return MFD_OK;
+        }
+        if (which == MFD_INT_E2) return read_integral(which, dst);
         if (which != MFD_INT_JE && which != MFD_INT_RHO) { err = "bad integral"; return MFD_ERR_INVALID; }
         const size_t es = which == MFD_INT_JE ? sizeof(T) : sizeof(double);
         // no plasma: zeros without touching the device, as mfd_read_integral returns them
@@ -2345,11 +2419,8 @@ struct mfd_batch {
         E* e;
         long long first, last, it;
         int flags;
-        HParams<float>* hp = nullptr;
-        EParams<float, double>* ep = nullptr;
-        MonParams<float>* mp = nullptr;
-        RectParams<float>* rp = nullptr;
         long long cells;
+        int slot = -1;   // its row in the tables
     };
     int dev = 0;
     cudaStream_t st = nullptr;
@@ -2358,6 +2429,12 @@ struct mfd_batch {
     std::vector<Member> mem;
     // tables
     DevBuf<BMember> d_mem;
+    DevBuf<HParams<float>> d_hp;           // the members' parameter blocks, by slot
+    DevBuf<EParams<float, double>> d_ep;
+    DevBuf<MonParams<float>> d_mp;
+    DevBuf<RectParams<float>> d_rp;
+    int table_n = 0;                       // rows of the tables
+    long long table_cells = 0, idle_cells = 0;   // cells of the members in the tables, and of those that finished
     DevBuf<BTile> d_tiles, d_tiles3;       // tiles of 2-D / 3-D members
     DevBuf<BMatTile> d_mtiles, d_mtiles3;
     DevBuf<BSrc> d_srcs;
@@ -2391,6 +2468,7 @@ struct mfd_batch {
         if (st) cudaStreamSynchronize(st);
         if (gexec) cudaGraphExecDestroy(gexec);
         for (auto& m : mem) release(m);
+        d_hp.release(); d_ep.release(); d_mp.release(); d_rp.release();
         d_mem.release(); d_tiles.release(); d_mtiles.release(); d_tiles3.release(); d_mtiles3.release();
         d_srcs.release(); d_mpts.release(); d_counts.release();
         d_spass.clear();
@@ -2401,21 +2479,7 @@ struct mfd_batch {
     }
 
     void release(Member& m) {
-        if (m.hp) cudaFreeAsync(m.hp, st);
-        if (m.ep) cudaFreeAsync(m.ep, st);
-        if (m.mp) cudaFreeAsync(m.mp, st);
-        if (m.rp) cudaFreeAsync(m.rp, st);
-        m.hp = nullptr; m.ep = nullptr; m.mp = nullptr; m.rp = nullptr;
         if (m.e) m.e->in_batch = false;
-    }
-
-    template <typename U>
-    U* copy_struct(const U& v) {
-        U* d = nullptr;
-        if (cudaMallocAsync(&d, sizeof(U), st) != cudaSuccess) { cudaGetLastError(); throw Error(MFD_ERR_OOM, "batch member allocation failed"); }
-        MFD_CK(cudaMemcpyAsync(d, &v, sizeof(U), cudaMemcpyHostToDevice, st));
-        MFD_CK(cudaStreamSynchronize(st));   // the host copy is a temporary
-        return d;
     }
 
     void init(int device) {
@@ -2448,15 +2512,6 @@ struct mfd_batch {
         m.flags = (e->math_needed ? BF_MATH : 0) | (e->any_geom ? BF_MAT : 0) | (e->fastdiv ? BF_FAST : 0) | (e->ndim == 3 ? BF_3D : 0) |
                   (e->recip ? BF_RECIP : 0);
         m.cells = (long long)e->nx * e->ny * e->nz;
-        try {
-            m.hp = copy_struct(e->hparams(0, 0));
-            m.ep = copy_struct(e->eparams());
-            m.mp = copy_struct(e->mon_p);
-            if (e->tfsf) m.rp = copy_struct(e->tfsf_p);
-        } catch (...) {
-            release(m);
-            throw;
-        }
         MFD_CK(cudaStreamSynchronize(e->st));          // the member's own work is complete
         MFD_CK(cudaEventRecord(e->run_ev[0], e->st));
         e->in_batch = true;
@@ -2468,6 +2523,16 @@ struct mfd_batch {
     // Tables of the current members and tile shape, then the graph of gsteps steps.
     void rebuild() {
         std::vector<BMember> hm;
+        std::vector<HParams<float>> hp;
+        std::vector<EParams<float, double>> ep;
+        std::vector<MonParams<float>> mp;
+        std::vector<RectParams<float>> rp(mem.size());
+        d_hp.reserve(mem.size(), st);
+        d_ep.reserve(mem.size(), st);
+        d_mp.reserve(mem.size(), st);
+        d_rp.reserve(mem.size(), st);
+        table_cells = idle_cells = 0;
+        table_n = (int)mem.size();
         std::vector<BTile> tiles, tiles3;
         std::vector<BMatTile> mt, mt3;
         std::vector<BSrc> srcs;
@@ -2477,10 +2542,16 @@ struct mfd_batch {
         std::vector<BPoint> mpts;
         has_set[0] = has_set[1] = false;
         for (size_t i = 0; i < mem.size(); ++i) {
-            const Member& m = mem[i];
+            Member& m = mem[i];
             E* e = m.e;
+            m.slot = (int)i;
+            table_cells += m.cells;
+            hp.push_back(e->hparams(0, 0));
+            ep.push_back(e->eparams());
+            mp.push_back(e->mon_p);
+            if (e->tfsf) rp[i] = e->tfsf_p;
             has_set[(m.flags & BF_RECIP) ? 1 : 0] = true;
-            hm.push_back(BMember{m.hp, m.ep, m.mp, m.rp, m.it, m.first, m.last, e->ring_first, m.flags, 0, e->d3});
+            hm.push_back(BMember{d_hp.p + i, d_ep.p + i, d_mp.p + i, e->tfsf ? d_rp.p + i : nullptr, m.it, m.first, m.last, e->ring_first, m.flags, 0, e->d3});
             const int mi = (int)i;
             const bool d3 = e->ndim == 3;
             const int rows = d3 ? e->ny * e->nz : e->nz;   // 3-D: rows y + ny z
@@ -2518,6 +2589,10 @@ struct mfd_batch {
                 for (long long j = 0; j < e->mons_host[k].npts; ++j) mpts.push_back(BPoint{mi, (int)k, j});
         }
         d_mem.upload(hm, st);
+        d_hp.upload(hp, st);
+        d_ep.upload(ep, st);
+        d_mp.upload(mp, st);
+        d_rp.upload(rp, st);
         d_tiles.upload(tiles, st);
         d_mtiles.upload(mt, st);
         d_tiles3.upload(tiles3, st);
@@ -2621,7 +2696,7 @@ struct mfd_batch {
                 batch_source_kernel<<<(spass_n[k] + 255) / 256, 256, 0, st>>>(d_mem.p, d_srcs.p, d_spass[k]->p, d_counts.p + 5 + k);
         }
         if (nmpts) batch_gather_kernel<<<(nmpts + 255) / 256, 256, 0, st>>>(d_mem.p, d_mpts.p, d_counts.p + 2);
-        batch_advance_kernel<<<((int)mem.size() + 255) / 256, 256, 0, st>>>(d_mem.p, (int)mem.size());
+        batch_advance_kernel<<<(table_n + 255) / 256, 256, 0, st>>>(d_mem.p, table_n);
     }
 
     void build_graph() {
@@ -2650,12 +2725,15 @@ struct mfd_batch {
             }
             if (e->ring_used == 0 && e->ring_first != m.it - 1) {
                 e->ring_first = m.it - 1;
-                MFD_CK(cudaMemcpyAsync(&d_mem.p[i].ring_first, &e->ring_first, sizeof(long long), cudaMemcpyHostToDevice, st));
+                MFD_CK(cudaMemcpyAsync(&d_mem.p[m.slot].ring_first, &e->ring_first, sizeof(long long), cudaMemcpyHostToDevice, st));
             }
         }
     }
 
-    // Retire members whose window is done: the end-of-run work of mfd_run on their streams.
+    // Retire members whose window is done: the end-of-run work of mfd_run on their streams.  The
+    // kernels skip a finished member by its step alone (they read nothing else of it), so its
+    // rows may stay in the tables; they are rebuilt, and the graph captured anew (1.2 ms for 32
+    // 2-D models), once the finished members hold a quarter of the tables' cells.
     void retire() {
         std::vector<Member> keep;
         for (auto& m : mem) {
@@ -2663,9 +2741,10 @@ struct mfd_batch {
             m.e->in_batch = false;
             m.e->finish(m.first, m.last);   // its status (NaN/Inf step) is kept by the handle
             release(m);
-            dirty = true;
+            idle_cells += m.cells;
         }
         mem.swap(keep);
+        if (4 * idle_cells >= table_cells) dirty = true;
     }
 
     int run(long long max_steps, int* n_active) {
