@@ -17,11 +17,12 @@
 
 #include "aux.cuh"
 #include "yee.cuh"
+#include "yee2d_quad.cuh"
 #include "yee3d_split.cuh"
 
 namespace mfd {
 
-enum { BF_MATH = 1, BF_MAT = 2, BF_FAST = 4, BF_3D = 8, BF_RECIP = 16 };
+enum { BF_MATH = 1, BF_MAT = 2, BF_FAST = 4, BF_3D = 8, BF_RECIP = 16, BF_K1 = 32, BF_RESP = 64 };
 
 // The half-step kernels come in two sets: DSET 0 runs the members of the exact arithmetic
 // (IEEE or the verified constant division), DSET 1 those of the tolerance mode (reciprocal
@@ -44,7 +45,9 @@ struct BMember {
     Div3 d3;                               // grid-spacing divisors of a 3-D member (div6)
 };
 
-struct BTile {      // cells x0 .. x0+blockDim.x-1 of rows z0 .. z0+blockDim.y-1 of member m
+// 2-D: cells x0 .. x0 + 4 blockDim.x - 1 (four per thread) of rows z0 .. z0 + blockDim.y - 1 of
+// member m.
+struct BTile {
     int m, x0, z0, w;  // 3-D linear tiles: (x0, z0, w) = (x, y, z) of the tile's first cell
 };
 
@@ -86,9 +89,17 @@ __device__ __forceinline__ void b_stage(P* dst, const P* src) {
 }
 
 
+// Entry of a block's k-th turn (runs of CHUNK consecutive tiles, dealt out to the blocks in turn);
+// m = -1 past the end.
+template <int CHUNK>
+__device__ __forceinline__ BTile b_tile(const BTile* __restrict__ tiles, int k, int n) {
+    const int t = ((k / CHUNK) * (int)gridDim.x + (int)blockIdx.x) * CHUNK + k % CHUNK;
+    if (t < n) return tiles[t];
+    return BTile{-1, 0, 0, 0};
+}
+
 #define MFD_B2D_CHUNK 4  // a block takes runs of this many consecutive tiles (fewer member changes)
-#define MFD_B2D_MINB 4   // batched 2-D updates: 4 blocks of 512 threads per SM (32 registers; the tolerance set's E
-                         // kernel spills 36 bytes there, and still measured 43.9 against 41.4 Gcell/s at 3 blocks)
+#define MFD_B2D_MINB 2   // batched 2-D updates: 2 blocks of 512 threads per SM (64 registers for four cells a thread)
 
 
 template <int DSET>
@@ -96,36 +107,42 @@ __global__ void __launch_bounds__(512, MFD_B2D_MINB) batch_h2d_kernel(const BMem
                                                         const int* __restrict__ ntiles) {
     __shared__ __align__(16) HParams<float> sp;
     const int n = *ntiles;
-    int cur = -1;
+    int cur = -1, acc = 0, flags = 0;
+    bool skip = false;
+    long long prev = 0;
     // Tile t of the block's k-th turn: runs of MFD_B2D_CHUNK tiles, the runs dealt out to the
-    // blocks in turn, so t grows with k.
-    for (int k = 0;; ++k) {
-        const int t = ((k / MFD_B2D_CHUNK) * (int)gridDim.x + (int)blockIdx.x) * MFD_B2D_CHUNK + k % MFD_B2D_CHUNK;
-        if (t >= n) break;
-        const BTile tl = tiles[t];
-        const BMember& M = mem[tl.m];
-        if (!b_active(M) || b_other_set<DSET>(M.flags)) continue;   // the same for the whole block
-        const int acc = M.it > M.first ? 1 : 0;
-        const long long prev = M.it - 1;
-        const int flags = M.flags;
+    // blocks in turn, so t grows with k.  The next turn's entry is fetched while this one runs,
+    // and the member's step and flags are read when the member changes.
+    BTile nxt = b_tile<MFD_B2D_CHUNK>(tiles, 0, n);
+    for (int k = 0; nxt.m >= 0; ++k) {
+        const BTile tl = nxt;
+        nxt = b_tile<MFD_B2D_CHUNK>(tiles, k + 1, n);
         if (tl.m != cur) {   // the block copies the member's parameters to shared memory (42.1 vs 40.8 Gcell/s)
-            __syncthreads();          // the previous member's parameters are no longer read
-            b_stage(&sp, M.hp);
-            __syncthreads();
+            const BMember& M = mem[tl.m];
             cur = tl.m;
+            flags = M.flags;
+            skip = !b_active(M) || b_other_set<DSET>(flags);   // the same for the whole block
+            acc = M.it > M.first ? 1 : 0;
+            prev = M.it - 1;
+            __syncthreads();          // the previous member's parameters are no longer read
+            if (!skip) b_stage(&sp, M.hp);
+            __syncthreads();
         }
+        if (skip) continue;
         const HParams<float>& p = sp;
-        const int ix = tl.x0 + threadIdx.x, iz = tl.z0 + threadIdx.y;
-        if (ix >= p.L.nx || iz >= p.L.nz) continue;
+        const int x0 = tl.x0 + 4 * (int)threadIdx.x, iz = tl.z0 + threadIdx.y;
+        if (x0 >= p.L.nx || iz >= p.L.nz) continue;
+        const bool k1 = flags & BF_K1;
         if constexpr (DSET == 1) {
-            if (flags & BF_MATH) h2d_cell<float, true, DIV_RECIP>(p, acc, prev, ix, iz);
-            else h2d_cell<float, false, DIV_RECIP>(p, acc, prev, ix, iz);
-        } else {
-            switch (flags & (BF_MATH | BF_FAST)) {
-                case 0: h2d_cell<float, false, DIV_IEEE>(p, acc, prev, ix, iz); break;
-                case BF_MATH: h2d_cell<float, true, DIV_IEEE>(p, acc, prev, ix, iz); break;
-                case BF_FAST: h2d_cell<float, false, DIV_EXACT>(p, acc, prev, ix, iz); break;
-                default: h2d_cell<float, true, DIV_EXACT>(p, acc, prev, ix, iz); break;
+            if (flags & BF_MATH) h2d_quad<true, DIV_RECIP>(p, k1, acc, prev, x0, iz);
+            else h2d_quad<false, DIV_RECIP>(p, k1, acc, prev, x0, iz);
+        } else if (flags & BF_FAST) {
+            if (flags & BF_MATH) h2d_quad<true, DIV_EXACT>(p, k1, acc, prev, x0, iz);
+            else h2d_quad<false, DIV_EXACT>(p, k1, acc, prev, x0, iz);
+        } else {   // a divisor that needs IEEE division: cell by cell
+            for (int ix = x0; ix < min(x0 + 4, p.L.nx); ++ix) {
+                if (flags & BF_MATH) h2d_cell<float, true, DIV_IEEE>(p, acc, prev, ix, iz);
+                else h2d_cell<float, false, DIV_IEEE>(p, acc, prev, ix, iz);
             }
         }
     }
@@ -136,34 +153,39 @@ __global__ void __launch_bounds__(512, MFD_B2D_MINB) batch_e2d_kernel(const BMem
                                                         const int* __restrict__ ntiles) {
     __shared__ __align__(16) EParams<float, double> sp;
     const int n = *ntiles;
-    int cur = -1;
-    // Tile t of the block's k-th turn: runs of MFD_B2D_CHUNK tiles, the runs dealt out to the
-    // blocks in turn, so t grows with k.
-    for (int k = 0;; ++k) {
-        const int t = ((k / MFD_B2D_CHUNK) * (int)gridDim.x + (int)blockIdx.x) * MFD_B2D_CHUNK + k % MFD_B2D_CHUNK;
-        if (t >= n) break;
-        const BTile tl = tiles[t];
-        const BMember& M = mem[tl.m];
-        if (!b_active(M) || b_other_set<DSET>(M.flags)) continue;   // the same for the whole block
-        const int flags = M.flags;
-        if (tl.m != cur) {   // the block copies the member's parameters to shared memory (42.1 vs 40.8 Gcell/s)
-            __syncthreads();
-            b_stage(&sp, M.ep);
-            __syncthreads();
+    int cur = -1, flags = 0, cur_p = 0;   // cur_p: ping-pong parity of the polarisation
+    bool skip = false;
+    BTile nxt = b_tile<MFD_B2D_CHUNK>(tiles, 0, n);   // as in the H kernel
+    for (int k = 0; nxt.m >= 0; ++k) {
+        const BTile tl = nxt;
+        nxt = b_tile<MFD_B2D_CHUNK>(tiles, k + 1, n);
+        if (tl.m != cur) {
+            const BMember& M = mem[tl.m];
             cur = tl.m;
+            flags = M.flags;
+            skip = !b_active(M) || b_other_set<DSET>(flags);   // the same for the whole block
+            cur_p = (int)((M.it - 1) & 1);
+            __syncthreads();
+            if (!skip) b_stage(&sp, M.ep);
+            __syncthreads();
         }
+        if (skip) continue;
         const EParams<float, double>& p = sp;
-        const int ix = tl.x0 + threadIdx.x, iz = tl.z0 + threadIdx.y;
-        if (ix >= p.L.nx || iz >= p.L.nz) continue;
+        const int x0 = tl.x0 + 4 * (int)threadIdx.x, iz = tl.z0 + threadIdx.y;
+        const bool act = x0 < p.L.nx && iz < p.L.nz;
+        const bool k1 = flags & BF_K1;
         if constexpr (DSET == 1) {
-            if (flags & BF_MAT) e2d_cell<float, double, true, DIV_RECIP>(p, ix, iz);
-            else e2d_cell<float, double, false, DIV_RECIP>(p, ix, iz);
-        } else {
-            switch (flags & (BF_MAT | BF_FAST)) {
-                case 0: e2d_cell<float, double, false, DIV_IEEE>(p, ix, iz); break;
-                case BF_MAT: e2d_cell<float, double, true, DIV_IEEE>(p, ix, iz); break;
-                case BF_FAST: e2d_cell<float, double, false, DIV_EXACT>(p, ix, iz); break;
-                default: e2d_cell<float, double, true, DIV_EXACT>(p, ix, iz); break;
+            if (flags & BF_RESP) e2d_warp<double, true, DIV_RECIP, true>(p, k1, cur_p, act, x0, iz);
+            else if (flags & BF_MAT) e2d_warp<double, true, DIV_RECIP, false>(p, k1, cur_p, act, x0, iz);
+            else e2d_warp<double, false, DIV_RECIP, false>(p, k1, cur_p, act, x0, iz);
+        } else if (flags & BF_FAST) {
+            if (flags & BF_RESP) e2d_warp<double, true, DIV_EXACT, true>(p, k1, cur_p, act, x0, iz);
+            else if (flags & BF_MAT) e2d_warp<double, true, DIV_EXACT, false>(p, k1, cur_p, act, x0, iz);
+            else e2d_warp<double, false, DIV_EXACT, false>(p, k1, cur_p, act, x0, iz);
+        } else if (act) {   // a divisor that needs IEEE division: cell by cell
+            for (int ix = x0; ix < min(x0 + 4, p.L.nx); ++ix) {
+                if (flags & BF_MAT) e2d_cell<float, double, true, DIV_IEEE>(p, ix, iz);
+                else e2d_cell<float, double, false, DIV_IEEE>(p, ix, iz);
             }
         }
     }

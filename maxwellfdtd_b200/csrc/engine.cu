@@ -28,6 +28,7 @@
 #include "aux.cuh"
 #include "dft_tc.cuh"
 #include "yee.cuh"
+#include "yee2d_quad.cuh"
 #include "yee3d_async.cuh"
 #include "yee3d_split.cuh"
 #include "batch.cuh"
@@ -1506,8 +1507,24 @@ class Engine : public HandleBase {
         return p;
     }
 
+    // Single-precision 2-D models of the first field set step four cells per thread
+    // (yee2d_quad.cuh) unless a divisor needs IEEE division; the material response then runs in
+    // the E update when every response material has at most three poles and no plasma.
+    bool quad2d() const { return sizeof(T) == 4 && ndim == 2 && !ey2 && (recip || fastdiv); }
+    bool quad_resp() const {
+        if (any_plasma) return false;
+        for (int g : response_mats)
+            if (mats_host[g - 1].nq > 3) return false;
+        return true;
+    }
     template <bool MATH, int FAST>
     void launch_H_t(const HParams<T>& p) {
+        if constexpr (sizeof(T) == 4 && FAST != DIV_IEEE) {
+            if (quad2d()) {
+                h2d_quad_kernel<MATH, FAST><<<dim3((nx + 127) / 128, (nz + Q_TY - 1) / Q_TY), dim3(32, Q_TY), 0, st>>>(p, kappa_one);
+                return;
+            }
+        }
         if (ndim == 3) {
             dim3 blk(bx3, by3), grd((nx + bx3 - 1) / bx3, (ny + by3 - 1) / by3, (nz + zc3 - 1) / zc3);
             h3d_kernel<T, MATH, FAST><<<grd, blk, 0, st>>>(p, zc3);
@@ -1758,7 +1775,15 @@ class Engine : public HandleBase {
     }
 
     template <bool MAT, int FAST>
-    void launch_E_t(const EParams<T, R>& p) {
+    void launch_E_t(const EParams<T, R>& p, int cur) {
+        if constexpr (sizeof(T) == 4 && FAST != DIV_IEEE) {
+            if (quad2d()) {
+                const dim3 grd((nx + 127) / 128, (nz + Q_TY - 1) / Q_TY), blk(32, Q_TY);
+                if (MAT && !response_mats.empty() && quad_resp()) e2d_quad_kernel<R, MAT, FAST, true><<<grd, blk, 0, st>>>(p, kappa_one, cur);
+                else e2d_quad_kernel<R, MAT, FAST, false><<<grd, blk, 0, st>>>(p, kappa_one, cur);
+                return;
+            }
+        }
         if (ndim == 3) {
             dim3 blk(bx3, by3), grd((nx + bx3 - 1) / bx3, (ny + by3 - 1) / by3, (nz + zc3 - 1) / zc3);
             e3d_kernel<T, R, MAT, FAST><<<grd, blk, 0, st>>>(p, zc3);
@@ -1802,13 +1827,14 @@ class Engine : public HandleBase {
             launch(KC_E, [&] {
                 with_div([&](auto dm) {
                     constexpr int D = decltype(dm)::value;
-                    if (any_geom) launch_E_t<true, D>(p);
-                    else launch_E_t<false, D>(p);
+                    if (any_geom) launch_E_t<true, D>(p, cur);
+                    else launch_E_t<false, D>(p, cur);
                 });
             });
         // E of dispersive / plasma / Kerr cells: material_flat_kernel for up to 3 poles,
         // material_kernel (poles in a runtime loop) beyond -- unless the E update did it
         if (ndim == 3 && use_split && resp_fused) return;
+        if (quad2d() && quad_resp()) return;
         for (int g : response_mats) {
             const MatDev<T, R>& m = mats_host[g - 1];
             launch(KC_MAT, [&] {
@@ -2510,7 +2536,8 @@ struct mfd_batch {
         Member m{};
         m.h = h; m.e = e; m.first = e->done + 1; m.last = last; m.it = m.first;
         m.flags = (e->math_needed ? BF_MATH : 0) | (e->any_geom ? BF_MAT : 0) | (e->fastdiv ? BF_FAST : 0) | (e->ndim == 3 ? BF_3D : 0) |
-                  (e->recip ? BF_RECIP : 0);
+                  (e->recip ? BF_RECIP : 0) | (e->kappa_one ? BF_K1 : 0) |
+                  (e->quad2d() && !e->response_mats.empty() && e->quad_resp() ? BF_RESP : 0);
         m.cells = (long long)e->nx * e->ny * e->nz;
         MFD_CK(cudaStreamSynchronize(e->st));          // the member's own work is complete
         MFD_CK(cudaEventRecord(e->run_ev[0], e->st));
@@ -2563,8 +2590,9 @@ struct mfd_batch {
                 }
             } else {
                 for (int z = 0; z < rows; z += cur_tz)
-                    for (int x = 0; x < e->nx; x += cur_tx) (d3 ? tiles3 : tiles).push_back(BTile{mi, x, z, 0});
+                    for (int x = 0; x < e->nx; x += 4 * cur_tx) tiles.push_back(BTile{mi, x, z, 0});
             }
+            if (!(m.flags & BF_RESP))   // else the E update takes the response
             for (int g : e->response_mats) {
                 const MatDev<float, double>& md = e->mats_host[g - 1];
                 const int y0 = d3 ? md.by0 : 0, y1 = d3 ? md.by0 + md.bny : 1;
