@@ -13,8 +13,10 @@
 // are bit-identical.
 //
 // Measured per step: 1801 x 1203 cells with Drude and Lorentz media, tolerance mode 57.6 us with
-// one cell per thread and the material kernel, 41.6 now (H 15 us for 69 MB: 4.6 TB/s); 32 batched
-// models of 128-1024 cells a side, exact mode 277 us, 262 now (latency: 45 % of the warps active).
+// one cell per thread and the material kernel, 37.1 now (41.6 with the psi loads after the first
+// stores; the batched kernels, which hold their parameters in shared memory, spill with them ahead:
+// 262 -> 287 us, so they keep them behind); 32 batched
+// models of 128-1024 cells a side, exact mode 277 us, 254 now (latency: 45 % of the warps active).
 #pragma once
 
 #include "yee.cuh"
@@ -94,8 +96,83 @@ __device__ __forceinline__ void q_face_z(const LayerDev<float>& l, bool right, b
     q_store(at, ps, nv);
 }
 
+// The same with the psi loads apart (a kernel with registers to spare):
+// One CPML face of four cells, x (Z false: it may hold some of the cells only, in: bits) or z: psi
+// row P of derivative d.  load() issues the psi loads with the group's field loads, before any
+// store; step() computes, stores and passes cell j's psi to field(j, psi).
+template <bool Z, int P>
+struct QFace {
+    unsigned in = 0;
+    int q, k;
+    float ps[4];
+
+    __device__ __forceinline__ void load(const LayerDev<float>& l, bool right, int px, int x0, int nv, int iz) {
+        in = 0;
+        if (!l.nb) return;
+        if constexpr (Z) {
+            if (right ? iz < l.ib - 1 : iz >= l.ib) return;
+            q = right ? iz - (l.ib - 1) : iz;
+            k = x0 + px * q;
+            in = 15u;
+            q_load(l.psi[P] + k, ps);
+        } else {
+            if (right ? x0 + nv <= l.ib - 1 : x0 >= l.ib) return;
+            q = right ? x0 - (l.ib - 1) : x0;   // of cell 0; may lie before the layer
+            k = q + l.nb * iz;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                ps[j] = 0.0f;
+                if (j < nv && (right ? q + j >= 0 : x0 + j < l.ib)) {
+                    in |= 1u << j;
+                    ps[j] = l.psi[P][k + j];
+                }
+            }
+        }
+    }
+
+    template <int FAST, typename F>
+    __device__ __forceinline__ void step(const LayerDev<float>& l, bool k1, int nv, float (&d)[4], F&& field) {
+        if (!in) return;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (!Z && !(in >> j & 1u)) continue;
+            const int qj = Z ? q : q + j;
+            ps[j] = l.B[qj] * ps[j] + l.A[qj] * d[j];
+            if (!Z) l.psi[P][k + j] = ps[j];
+            field(j, ps[j]);
+            if (!k1) d[j] = cdiv<FAST>(d[j], l.K[qj]);
+        }
+        if (Z) q_store(l.psi[P] + k, ps, nv);
+    }
+};
+
+// Both faces of an axis.  A group in both of them (it spans the gap of two x layers, or the layers
+// overlap) loads the right one's psi after the left one's step.
+template <bool Z, int P>
+struct QAxis {
+    QFace<Z, P> f;
+    bool right;
+    __device__ __forceinline__ void load(const LayerDev<float>& l, const LayerDev<float>& r, int px, int x0, int nv, int iz) {
+        right = false;
+        f.load(l, false, px, x0, nv, iz);
+        if (!f.in) {
+            right = true;
+            f.load(r, true, px, x0, nv, iz);
+        }
+    }
+    template <int FAST, typename F>
+    __device__ __forceinline__ void step(const LayerDev<float>& l, const LayerDev<float>& r, int px, bool k1, int x0, int nv, int iz,
+                                         float (&d)[4], F&& field) {
+        f.template step<FAST>(right ? r : l, k1, nv, d, field);
+        if (!right && f.in && r.nb) {
+            f.load(r, true, px, x0, nv, iz);
+            f.template step<FAST>(r, k1, nv, d, field);
+        }
+    }
+};
+
 // Cells x0 .. x0 + 3 of row iz (x0 a multiple of 4 below nx).  k1: every kappa is 1.
-template <bool MATH, int FAST>
+template <bool MATH, int FAST, bool PRE = false>
 __device__ __forceinline__ void h2d_quad(const HParams<float>& p, bool k1, int accum, long long prev_step, int x0, int iz) {
     const int nx = p.L.nx, nz = p.L.nz, sz = p.L.sz;
     const int nv = min(4, nx - x0);
@@ -114,6 +191,12 @@ __device__ __forceinline__ void h2d_quad(const HParams<float>& p, bool k1, int a
     ez[4] = p.Ez[c + (!xr ? 4 : bx == MFD_BC_PERIODIC ? -x0 : nv - 1)];
     q_load(p.Ex + (c + (!zr ? sz : bz == MFD_BC_PERIODIC ? -(nz - 1) * sz : 0)), up);
     q_load(p.Hy + c, hy);
+    QAxis<false, 1> X;
+    QAxis<true, 1> Z;
+    if (PRE) {
+        X.load(p.lay[MFD_XL], p.lay[MFD_XR], p.L.px, x0, nv, iz);
+        Z.load(p.lay[MFD_ZL], p.lay[MFD_ZR], p.L.px, x0, nv, iz);
+    }
     if (accum) {
         q_load(p.Sa + c, sa);
         if (p.sum_e2) q_load(p.E2 + c, e2);
@@ -157,10 +240,15 @@ __device__ __forceinline__ void h2d_quad(const HParams<float>& p, bool k1, int a
     q_div<FAST>(p.ddx, n, dx);
     auto plus = [&](int j, float ps) { hy[j] = mad<FAST>(Mh[j], ps, hy[j]); };
     auto minus = [&](int j, float ps) { hy[j] = mad<FAST>(-Mh[j], ps, hy[j]); };
-    q_face_x<1, FAST>(p.lay[MFD_XL], false, k1, x0, nv, iz, dx, plus);
-    q_face_x<1, FAST>(p.lay[MFD_XR], true, k1, x0, nv, iz, dx, plus);
-    q_face_z<1, FAST>(p.lay[MFD_ZL], false, k1, p.L.px, x0, nv, iz, dz, minus);
-    q_face_z<1, FAST>(p.lay[MFD_ZR], true, k1, p.L.px, x0, nv, iz, dz, minus);
+    if constexpr (PRE) {
+        X.template step<FAST>(p.lay[MFD_XL], p.lay[MFD_XR], p.L.px, k1, x0, nv, iz, dx, plus);
+        Z.template step<FAST>(p.lay[MFD_ZL], p.lay[MFD_ZR], p.L.px, k1, x0, nv, iz, dz, minus);
+    } else {
+        q_face_x<1, FAST>(p.lay[MFD_XL], false, k1, x0, nv, iz, dx, plus);
+        q_face_x<1, FAST>(p.lay[MFD_XR], true, k1, x0, nv, iz, dx, plus);
+        q_face_z<1, FAST>(p.lay[MFD_ZL], false, k1, p.L.px, x0, nv, iz, dz, minus);
+        q_face_z<1, FAST>(p.lay[MFD_ZR], true, k1, p.L.px, x0, nv, iz, dz, minus);
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) hy[j] = mad<FAST>(-Mh[j], dz[j] - dx[j], hy[j]);
     q_store(p.Hy + c, hy, nv);
@@ -191,7 +279,7 @@ __device__ __forceinline__ void q_response(const EParams<float, R>& p, int x0w, 
 }
 
 // Returns whether some cell's E is left to the material response.
-template <typename R, bool MAT, int FAST>
+template <typename R, bool MAT, int FAST, bool PRE>
 __device__ __forceinline__ bool e2d_quad(const EParams<float, R>& p, bool k1, int x0, int iz) {
     const int nx = p.L.nx, nz = p.L.nz, sz = p.L.sz;
     const int c = x0 + sz * iz;
@@ -204,6 +292,12 @@ __device__ __forceinline__ bool e2d_quad(const EParams<float, R>& p, bool k1, in
     q_load(p.Hy + (c + (!zl ? -sz : bz == MFD_BC_PERIODIC ? (nz - 1) * sz : 0)), dn);
     q_load(p.Dx + c, D0);
     q_load(p.Dz + c, D2);
+    QAxis<false, 0> X;
+    QAxis<true, 0> Z;
+    if (PRE) {
+        X.load(p.lay[MFD_XL], p.lay[MFD_XR], p.L.px, x0, nv, iz);
+        Z.load(p.lay[MFD_ZL], p.lay[MFD_ZR], p.L.px, x0, nv, iz);
+    }
     uchar4 g4 = make_uchar4(0, 0, 0, 0);
     if (MAT) g4 = *reinterpret_cast<const uchar4*>(p.geom + c);
     if (xl && bx == MFD_BC_DIRICHLET) left = 0.0f;
@@ -235,10 +329,15 @@ __device__ __forceinline__ bool e2d_quad(const EParams<float, R>& p, bool k1, in
     q_div<FAST>(p.ddz, n, dz);
     auto plus = [&](int j, float ps) { D2[j] = mad<FAST>(Md2[j], ps, D2[j]); };
     auto minus = [&](int j, float ps) { D0[j] = mad<FAST>(-Md2[j], ps, D0[j]); };
-    q_face_x<0, FAST>(p.lay[MFD_XL], false, k1, x0, nv, iz, dx, plus);
-    q_face_x<0, FAST>(p.lay[MFD_XR], true, k1, x0, nv, iz, dx, plus);
-    q_face_z<0, FAST>(p.lay[MFD_ZL], false, k1, p.L.px, x0, nv, iz, dz, minus);
-    q_face_z<0, FAST>(p.lay[MFD_ZR], true, k1, p.L.px, x0, nv, iz, dz, minus);
+    if constexpr (PRE) {
+        X.template step<FAST>(p.lay[MFD_XL], p.lay[MFD_XR], p.L.px, k1, x0, nv, iz, dx, plus);
+        Z.template step<FAST>(p.lay[MFD_ZL], p.lay[MFD_ZR], p.L.px, k1, x0, nv, iz, dz, minus);
+    } else {
+        q_face_x<0, FAST>(p.lay[MFD_XL], false, k1, x0, nv, iz, dx, plus);
+        q_face_x<0, FAST>(p.lay[MFD_XR], true, k1, x0, nv, iz, dx, plus);
+        q_face_z<0, FAST>(p.lay[MFD_ZL], false, k1, p.L.px, x0, nv, iz, dz, minus);
+        q_face_z<0, FAST>(p.lay[MFD_ZR], true, k1, p.L.px, x0, nv, iz, dz, minus);
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         D0[j] = Md1[j] * D0[j] + Md2[j] * (0.0f - dz[j]);
@@ -267,9 +366,9 @@ __device__ __forceinline__ bool e2d_quad(const EParams<float, R>& p, bool k1, in
 
 // The E update of a warp's groups (every lane of the warp calls it; act: the lane's group lies in
 // the grid).  RESP: with the material response (else a material kernel follows).
-template <typename R, bool MAT, int FAST, bool RESP>
+template <typename R, bool MAT, int FAST, bool RESP, bool PRE = false>
 __device__ __forceinline__ void e2d_warp(const EParams<float, R>& p, bool k1, int cur, bool act, int x0, int iz) {
-    const bool resp = act && e2d_quad<R, MAT, FAST>(p, k1, x0, iz);
+    const bool resp = act && e2d_quad<R, MAT, FAST, PRE>(p, k1, x0, iz);
     if constexpr (MAT && RESP) {
         if (__any_sync(0xffffffffu, resp)) {
             __syncwarp();
@@ -284,13 +383,13 @@ constexpr int Q_TY = 8;
 template <bool MATH, int FAST>
 __global__ void __launch_bounds__(32 * Q_TY, 4) h2d_quad_kernel(const __grid_constant__ HParams<float> p, const bool k1) {
     const int x0 = 4 * (blockIdx.x * 32 + threadIdx.x), iz = blockIdx.y * Q_TY + threadIdx.y;
-    if (x0 < p.L.nx && iz < p.L.nz) h2d_quad<MATH, FAST>(p, k1, p.accum, p.prev_step, x0, iz);
+    if (x0 < p.L.nx && iz < p.L.nz) h2d_quad<MATH, FAST, true>(p, k1, p.accum, p.prev_step, x0, iz);
 }
 
 template <typename R, bool MAT, int FAST, bool RESP>
 __global__ void __launch_bounds__(32 * Q_TY, 4) e2d_quad_kernel(const __grid_constant__ EParams<float, R> p, const bool k1, const int cur) {
     const int x0 = 4 * (blockIdx.x * 32 + threadIdx.x), iz = blockIdx.y * Q_TY + threadIdx.y;
-    e2d_warp<R, MAT, FAST, RESP>(p, k1, cur, x0 < p.L.nx && iz < p.L.nz, x0, iz);
+    e2d_warp<R, MAT, FAST, RESP, true>(p, k1, cur, x0 < p.L.nx && iz < p.L.nz, x0, iz);
 }
 
 }  // namespace mfd
