@@ -399,7 +399,7 @@ __device__ __forceinline__ void material_cell(const MatDev<T, R>* __restrict__ m
         } else if (m->rate_kind == MFD_RATE_POWER) {
             T lg = log10(II);
             T a = m->rate_order * lg;
-            double R1 = pow(10.0, (double)a + m->rate_log10c);
+            const double R1 = exp10((double)a + m->rate_log10c);   // at most 1 ulp off; pow at most 2, and 150 instructions longer
             plasma_density<T, R, double>(rho, drho, R1, m->Rava * E2, dt);
         } else {
             plasma_density<T, R, T>(rho, drho, T(0), m->Rava * E2, dt);
@@ -505,7 +505,7 @@ __device__ __forceinline__ void material_cell_n(const MatDev<T, R>* __restrict__
         } else if (m->rate_kind == MFD_RATE_POWER) {
             T lg = log10(II);
             T a = m->rate_order * lg;
-            double R1 = pow(10.0, (double)a + m->rate_log10c);
+            const double R1 = exp10((double)a + m->rate_log10c);   // at most 1 ulp off; pow at most 2, and 150 instructions longer
             plasma_density<T, R, double>(rho, drho, R1, m->Rava * E2, dt);
         } else {
             plasma_density<T, R, T>(rho, drho, T(0), m->Rava * E2, dt);

@@ -947,11 +947,11 @@ __global__ void __launch_bounds__(256) material_flat_kernel(const MatDev<T, R>* 
     const long long bi = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (bi >= m->bsize) return;
     const int bnx = m->bnx, bny = m->bny;
-    const long long row = bi / bnx;
-    const int bx = (int)(bi - row * bnx);
-    const long long bz = row / bny;
-    const int by = (int)(row - bz * bny);
-    const int ix = m->bx0 + bx, iy = m->by0 + by, iz = m->bz0 + (int)bz;
+    const unsigned row = (unsigned)bi / (unsigned)bnx;   // a box has fewer than 2^31 cells
+    const int bx = (int)((unsigned)bi - row * (unsigned)bnx);
+    const int bz = (int)(row / (unsigned)bny);
+    const int by = (int)row - bz * bny;
+    const int ix = m->bx0 + bx, iy = m->by0 + by, iz = m->bz0 + bz;
     const int c = ix + L.px * iy + L.sz * iz;
     if (geom[c] != g) return;
     T Dv[NC];
