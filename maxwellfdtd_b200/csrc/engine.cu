@@ -346,6 +346,7 @@ class Engine : public HandleBase {
     T* matMh = nullptr;
     MatDev<T, R>* mats_dev = nullptr;
     std::vector<MatDev<T, R>> mats_host;
+    std::vector<bool> mat_full;       // the material fills its bounding box
     std::vector<int> response_mats;   // present materials whose E comes from material_kernel
     bool any_plasma = false;
 
@@ -580,7 +581,7 @@ class Engine : public HandleBase {
     // each material's bounding box read back for the compact state.  geom stays allocated
     // only when some cell holds a material.
     void device_geometry(const mfd_desc* d, std::vector<int>& bx0, std::vector<int>& bx1, std::vector<int>& by0,
-                         std::vector<int>& by1, std::vector<int>& bz0, std::vector<int>& bz1) {
+                         std::vector<int>& by1, std::vector<int>& bz0, std::vector<int>& bz1, std::vector<long long>& cnt) {
         if (d->geometry) throw Error(MFD_ERR_INVALID, "give either a geometry array or shapes, not both");
         if (!d->shapes || !d->coords[2] || (ndim >= 2 && !d->coords[0]) || (ndim == 3 && !d->coords[1]))
             throw Error(MFD_ERR_INVALID, "shapes need the shape list and the grid coordinates");
@@ -594,19 +595,20 @@ class Engine : public HandleBase {
         const double* ys = ndim == 3 ? upload(d->coords[1], (size_t)ny) : nullptr;
         const double* zs = upload(d->coords[2], (size_t)nz);
         geom = dalloc<uint8_t>((size_t)Np, false);
-        std::vector<int> box(6 * (size_t)nmat);
+        std::vector<int> box(7 * (size_t)nmat, 0);   // the boxes, then the cell counts
         for (int g = 0; g < nmat; ++g)
             for (int k = 0; k < 6; ++k) box[6 * g + k] = (k % 2) ? -1 : INT32_MAX;
         int* dbox = upload(box.data(), box.size());
         const long long nblk = ((long long)ny * nz + GEO_TY - 1) / GEO_TY;
         geometry_kernel<<<(unsigned)std::min(nblk, 148ll * 8), dim3(32, GEO_TY), 0, st>>>(geom, layout(), ds, d->nshape, xs, ys, zs,
-                                                                                        dbox, std::min(nmat, 255));
+                                                                                        dbox, dbox + 6 * (size_t)nmat, std::min(nmat, 255));
         MFD_CK(cudaGetLastError());
         MFD_CK(cudaMemcpyAsync(box.data(), dbox, box.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
         MFD_CK(cudaStreamSynchronize(st));
         for (int g = 1; g <= nmat; ++g) {
             const int* b = box.data() + 6 * (g - 1);
             bx0[g] = b[0]; bx1[g] = b[1]; by0[g] = b[2]; by1[g] = b[3]; bz0[g] = b[4]; bz1[g] = b[5];
+            cnt[g] = box[6 * (size_t)nmat + g - 1];
             if (b[1] >= 0) any_geom = true;
         }
     }
@@ -652,6 +654,7 @@ class Engine : public HandleBase {
         nmat = d->nmat;
         std::vector<int> bx0(nmat + 1, INT32_MAX), bx1(nmat + 1, -1), by0(nmat + 1, INT32_MAX), by1(nmat + 1, -1),
             bz0(nmat + 1, INT32_MAX), bz1(nmat + 1, -1);
+        std::vector<long long> cnt(nmat + 1, 0);   // cells of each material
         if (d->geometry) {
             // each material's bounding box, z-planes split over host threads (per-thread
             // boxes merged after); the map goes to its padded device layout in one 2-D copy
@@ -661,6 +664,7 @@ class Engine : public HandleBase {
             parallel_ranges(nz, 4, [&](long long z0, long long z1) {
                 std::vector<int> a0(nmat + 1, INT32_MAX), a1(nmat + 1, -1), b0(nmat + 1, INT32_MAX), b1(nmat + 1, -1),
                     c0(nmat + 1, INT32_MAX), c1(nmat + 1, -1);
+                std::vector<long long> n(nmat + 1, 0);
                 bool any = false, over = false;
                 for (int iz = (int)z0; iz < (int)z1; ++iz)
                     for (int iy = 0; iy < ny; ++iy) {
@@ -673,6 +677,7 @@ class Engine : public HandleBase {
                             if (!g) continue;
                             if (g > nmat) { over = true; continue; }
                             any = true;
+                            ++n[g];
                             a0[g] = std::min(a0[g], ix); a1[g] = std::max(a1[g], ix);
                             b0[g] = std::min(b0[g], iy); b1[g] = std::max(b1[g], iy);
                             c0[g] = std::min(c0[g], iz); c1[g] = std::max(c1[g], iz);
@@ -682,6 +687,7 @@ class Engine : public HandleBase {
                 bad = bad || over;
                 any_geom = any_geom || any;
                 for (int g = 1; g <= nmat; ++g) {
+                    cnt[g] += n[g];
                     bx0[g] = std::min(bx0[g], a0[g]); bx1[g] = std::max(bx1[g], a1[g]);
                     by0[g] = std::min(by0[g], b0[g]); by1[g] = std::max(by1[g], b1[g]);
                     bz0[g] = std::min(bz0[g], c0[g]); bz1[g] = std::max(bz1[g], c1[g]);
@@ -689,7 +695,7 @@ class Engine : public HandleBase {
             });
             if (bad) throw Error(MFD_ERR_INVALID, "geometry index beyond nmat");
         } else if (d->nshape > 0) {
-            device_geometry(d, bx0, bx1, by0, by1, bz0, bz1);
+            device_geometry(d, bx0, bx1, by0, by1, bz0, bz1, cnt);
         }
         if (d->geometry || d->nshape > 0) {
             for (int g = 1; g <= nmat; ++g) {
@@ -731,6 +737,8 @@ class Engine : public HandleBase {
                 M.bx0 = bx0[g]; M.by0 = by0[g]; M.bz0 = bz0[g];
                 M.bnx = bx1[g] - bx0[g] + 1; M.bny = by1[g] - by0[g] + 1; M.bnz = bz1[g] - bz0[g] + 1;
                 M.bsize = (long long)M.bnx * M.bny * M.bnz;
+                mat_full.resize(nmat, false);
+                mat_full[m] = cnt[g] == M.bsize;
             }
             if (present && M.nq > 0) M.P = dalloc<T>((size_t)2 * M.nq * nc * M.bsize);
             if (M.plasma) {
@@ -1864,6 +1872,7 @@ class Engine : public HandleBase {
     template <int NC>
     void launch_mat_flat(int g, const MatDev<T, R>& m, int cur) {
         const unsigned blocks = (unsigned)((m.bsize + 255) / 256);
+        const bool full = mat_full[g - 1];
         // NC = 3: x, y, z; 2: x, z; 1: the one component (Dy, Ey of the second 2-D field set)
         T* D0 = NC == 1 ? F[MFD_DY] : F[MFD_DX];
         T* E0 = NC == 1 ? F[MFD_EY] : F[MFD_EX];
@@ -1872,10 +1881,10 @@ class Engine : public HandleBase {
         T* Dz = NC == 1 ? nullptr : F[MFD_DZ];
         T* Ez = NC == 1 ? nullptr : F[MFD_EZ];
         switch (m.nq) {
-            case 0: material_flat_kernel<T, R, NC, 0><<<blocks, 256, 0, st>>>(mats_dev, g, geom, layout(), D0, Dy, Dz, E0, Ey, Ez, cur, dt); break;
-            case 1: material_flat_kernel<T, R, NC, 1><<<blocks, 256, 0, st>>>(mats_dev, g, geom, layout(), D0, Dy, Dz, E0, Ey, Ez, cur, dt); break;
-            case 2: material_flat_kernel<T, R, NC, 2><<<blocks, 256, 0, st>>>(mats_dev, g, geom, layout(), D0, Dy, Dz, E0, Ey, Ez, cur, dt); break;
-            default: material_flat_kernel<T, R, NC, 3><<<blocks, 256, 0, st>>>(mats_dev, g, geom, layout(), D0, Dy, Dz, E0, Ey, Ez, cur, dt); break;
+            case 0: material_flat_kernel<T, R, NC, 0><<<blocks, 256, 0, st>>>(m, g, full, geom, layout(), D0, Dy, Dz, E0, Ey, Ez, cur, dt); break;
+            case 1: material_flat_kernel<T, R, NC, 1><<<blocks, 256, 0, st>>>(m, g, full, geom, layout(), D0, Dy, Dz, E0, Ey, Ez, cur, dt); break;
+            case 2: material_flat_kernel<T, R, NC, 2><<<blocks, 256, 0, st>>>(m, g, full, geom, layout(), D0, Dy, Dz, E0, Ey, Ez, cur, dt); break;
+            default: material_flat_kernel<T, R, NC, 3><<<blocks, 256, 0, st>>>(m, g, full, geom, layout(), D0, Dy, Dz, E0, Ey, Ez, cur, dt); break;
         }
     }
 

@@ -42,8 +42,8 @@ __host__ __device__ __forceinline__ bool shape_covers(const mfd_shape& s, double
 }
 
 // The padded map (x fastest) and, in the same pass, the bounding box of each material's cells:
-// box[6 (g - 1) + {0..5}] = x0, x1, y0, y1, z0, z1 (initialised to INT_MAX / -1).  1-D and 2-D
-// grids take the missing coordinates as 0 (2-D: y; 1-D: x and y).
+// box[6 (g - 1) + {0..5}] = x0, x1, y0, y1, z0, z1 (initialised to INT_MAX / -1), and their number,
+// count[g - 1].  1-D and 2-D grids take the missing coordinates as 0 (2-D: y; 1-D: x and y).
 //
 // A warp walks rows 32 cells at a time.  The lanes of one material are found with a ballot, so
 // a segment gives at most one candidate interval per material; it is merged into the block's
@@ -57,10 +57,11 @@ constexpr int GEO_TY = 8;
 __global__ void __launch_bounds__(32 * GEO_TY) geometry_kernel(uint8_t* __restrict__ geom, const Layout L,
                                                                const mfd_shape* __restrict__ shapes, const int nshape,
                                                                const double* __restrict__ xs, const double* __restrict__ ys,
-                                                               const double* __restrict__ zs, int* box, const int nmat) {
-    __shared__ int sb[6 * 255];
+                                                               const double* __restrict__ zs, int* box, int* count, const int nmat) {
+    __shared__ int sb[6 * 255], sc[255];
     const int lane = threadIdx.x, tid = threadIdx.x + 32 * threadIdx.y;
     for (int i = tid; i < 6 * nmat; i += 32 * GEO_TY) sb[i] = (i & 1) ? -1 : 0x7fffffff;
+    for (int i = tid; i < nmat; i += 32 * GEO_TY) sc[i] = 0;
     __syncthreads();
     const long long rows = (long long)L.ny * L.nz;
     for (long long row = (long long)blockIdx.x * GEO_TY + threadIdx.y; row < rows; row += (long long)gridDim.x * GEO_TY) {
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(32 * GEO_TY) geometry_kernel(uint8_t* __restri
                     if (iy > b[3]) atomicMax(b + 3, iy);
                     if (iz < b[4]) atomicMin(b + 4, iz);
                     if (iz > b[5]) atomicMax(b + 5, iz);
+                    atomicAdd(&sc[gl - 1], __popc(m));
                 }
                 todo &= ~m;
             }
@@ -100,6 +102,8 @@ __global__ void __launch_bounds__(32 * GEO_TY) geometry_kernel(uint8_t* __restri
         if (i & 1) { if (sb[i] >= 0) atomicMax(box + i, sb[i]); }
         else if (sb[i] != 0x7fffffff) atomicMin(box + i, sb[i]);
     }
+    for (int i = tid; i < nmat; i += 32 * GEO_TY)
+        if (sc[i]) atomicAdd(count + i, sc[i]);
 }
 
 }  // namespace mfd
