@@ -10,7 +10,7 @@
 // e2d_cell, the 3-D h3d_cell / e3d_cell of the CPML slabs, material_cell, the point-source
 // expression), so a member's results are bit-identical to running it alone.  2-D and 3-D
 // members have their own tile tables and kernels (the 3-D cell code needs more registers);
-// a 3-D tile covers x cells by (y, z) rows numbered y + ny z.  A block copies its tile's
+// a 3-D tile is a run of groups of B3D_W cells.  A block copies its tile's
 // member parameter block into shared memory whenever the member changes, so the cells read
 // the layout, pointers and coefficients from there rather than through dependent global loads.
 #pragma once
@@ -18,6 +18,7 @@
 #include "aux.cuh"
 #include "yee.cuh"
 #include "yee2d_quad.cuh"
+#include "yee3d_group.cuh"
 #include "yee3d_split.cuh"
 
 namespace mfd {
@@ -48,7 +49,7 @@ struct BMember {
 // 2-D: cells x0 .. x0 + 4 blockDim.x - 1 (four per thread) of rows z0 .. z0 + blockDim.y - 1 of
 // member m.
 struct BTile {
-    int m, x0, z0, w;  // 3-D linear tiles: (x0, z0, w) = (x, y, z) of the tile's first cell
+    int m, x0, z0, w;  // 3-D linear tiles: (x0, z0, w) = (group of the row, y, z) of the tile's first group
 };
 
 struct BMatTile {   // one row segment of material g's bounding box: x0 .. x0+blockDim.x-1 at (iy, iz)
@@ -220,118 +221,118 @@ __global__ void __launch_bounds__(128) batch_material2d_kernel(const BMember* __
     }
 }
 
-#define MFD_B3D_MINB 3   // batched 3-D updates held to 40 registers (measured 16.0 against 15.0 Gcell/s at 58)
+// Cells of a 3-D thread's group: two, which fit 64 registers.  32 models of 48-128 cells a side,
+// tolerance mode: one cell 909 us per step, two 734, four (96-124 registers, a quarter of the
+// warps) 856.
+constexpr int B3D_W = 2;
 
-
-// The cell of a 3-D tile's thread.  A 3-D tile is a run of cells in x-fastest order (no
-// idle lanes at rows shorter than the block): the block's threads take the
-// blockDim.x * blockDim.y cells from the tile's first cell (x0, z0, w) = (x, y, z).
-__device__ __forceinline__ bool b_cell3(const Layout& L, const BTile& tl, int& ix, int& iy, int& iz) {
-    // offset / nx row steps, a few at the tile shapes used: cheaper than two divisions
-    ix = tl.x0 + (int)(threadIdx.y * blockDim.x + threadIdx.x);
+// The group of a 3-D tile's thread.  A 3-D tile is a run of groups in x-fastest order (no idle
+// lanes at rows shorter than the block): the block's threads take the blockDim.x * blockDim.y
+// groups from the tile's first, (x0, z0, w) = (group of the row, y, z).
+__device__ __forceinline__ bool b_group3(const Layout& L, const BTile& tl, int& x0, int& iy, int& iz) {
+    // offset / row length row steps, a few at the tile shapes used: cheaper than two divisions
+    const int ng = (L.nx + B3D_W - 1) / B3D_W;
+    x0 = tl.x0 + (int)(threadIdx.y * blockDim.x + threadIdx.x);
     iy = tl.z0;
     iz = tl.w;
-    while (ix >= L.nx) {
-        ix -= L.nx;
+    while (x0 >= ng) {
+        x0 -= ng;
         if (++iy == L.ny) {
             iy = 0;
             ++iz;
         }
     }
+    x0 *= B3D_W;
     return iz < L.nz;
 }
 
-#define MFD_B3D_CHUNK 16 // a block takes runs of this many consecutive tiles (fewer member changes)
-
-
-// The running sums of the previous step are added from a member's second step on.
-template <bool MATH, int FAST>
-__device__ __forceinline__ void b_h3d_p(const HParams<float>& p, const Div3& d3, long long it, long long first, int ix, int iy,
-                                        int iz) {
-    if (it == first) h3d_cell<float, MATH, FAST, false, false>(p, d3, it - 1, ix, iy, iz);
-    else if (p.sum_e2) h3d_cell<float, MATH, FAST, true, true>(p, d3, it - 1, ix, iy, iz);
-    else h3d_cell<float, MATH, FAST, true, false>(p, d3, it - 1, ix, iy, iz);
-}
+// A block takes runs of this many consecutive tiles (fewer member changes).  Runs of 2: 734 us; of 1
+// 764, 4 759-777, 8 808, 16 888.
+#define MFD_B3D_CHUNK 2
 
 template <int DSET>
-__global__ void __launch_bounds__(512, MFD_B3D_MINB) batch_h3d_kernel(const BMember* __restrict__ mem, const BTile* __restrict__ tiles,
-                                                        const int* __restrict__ ntiles) {
+__global__ void __launch_bounds__(512, 2) batch_h3d_kernel(const BMember* __restrict__ mem, const BTile* __restrict__ tiles,
+                                                           const int* __restrict__ ntiles) {
     __shared__ __align__(16) HParams<float> sp;
     __shared__ Div3 sd3;
     const int n = *ntiles;
-    int cur = -1;
-    // Tile t of the block's k-th turn: runs of MFD_B3D_CHUNK tiles, the runs dealt out to the
-    // blocks in turn, so t grows with k.
-    for (int k = 0;; ++k) {
-        const int t = ((k / MFD_B3D_CHUNK) * (int)gridDim.x + (int)blockIdx.x) * MFD_B3D_CHUNK + k % MFD_B3D_CHUNK;
-        if (t >= n) break;
-        const BTile tl = tiles[t];
-        const BMember& M = mem[tl.m];
-        if (!b_active(M) || b_other_set<DSET>(M.flags)) continue;   // the same for the whole block
-        const long long it = M.it, first = M.first;
-        const int flags = M.flags;
+    int cur = -1, flags = 0;
+    bool skip = false, acc = false;
+    long long prev = 0;
+    BTile nxt = b_tile<MFD_B3D_CHUNK>(tiles, 0, n);   // as in the 2-D kernels
+    for (int k = 0; nxt.m >= 0; ++k) {
+        const BTile tl = nxt;
+        nxt = b_tile<MFD_B3D_CHUNK>(tiles, k + 1, n);
         if (tl.m != cur) {   // the block copies the member's parameters to shared memory
-            __syncthreads();          // the previous member's parameters are no longer read
-            b_stage(&sp, M.hp);
-            if (threadIdx.x == 0 && threadIdx.y == 0) sd3 = M.d3;
-            __syncthreads();
+            const BMember& M = mem[tl.m];
             cur = tl.m;
-        }
-        const HParams<float>& p = sp;
-        const Div3& d3 = sd3;
-        int ix, iy, iz;
-        if (!b_cell3(p.L, tl, ix, iy, iz)) continue;
-        if constexpr (DSET == 1) {
-            if (flags & BF_MATH) b_h3d_p<true, DIV_RECIP>(p, d3, it, first, ix, iy, iz);
-            else b_h3d_p<false, DIV_RECIP>(p, d3, it, first, ix, iy, iz);
-        } else {
-            switch (flags & (BF_MATH | BF_FAST)) {
-                case 0: b_h3d_p<false, DIV_IEEE>(p, d3, it, first, ix, iy, iz); break;
-                case BF_MATH: b_h3d_p<true, DIV_IEEE>(p, d3, it, first, ix, iy, iz); break;
-                case BF_FAST: b_h3d_p<false, DIV_EXACT>(p, d3, it, first, ix, iy, iz); break;
-                default: b_h3d_p<true, DIV_EXACT>(p, d3, it, first, ix, iy, iz); break;
+            flags = M.flags;
+            skip = !b_active(M) || b_other_set<DSET>(flags);   // the same for the whole block
+            acc = M.it > M.first;    // the running sums of the previous step, from a member's second step on
+            prev = M.it - 1;
+            __syncthreads();          // the previous member's parameters are no longer read
+            if (!skip) {
+                b_stage(&sp, M.hp);
+                if (threadIdx.x == 0 && threadIdx.y == 0) sd3 = M.d3;
             }
+            __syncthreads();
+        }
+        if (skip) continue;
+        const HParams<float>& p = sp;
+        int x0, iy, iz;
+        if (!b_group3(p.L, tl, x0, iy, iz)) continue;
+        const bool k1 = flags & BF_K1;
+        if constexpr (DSET == 1) {
+            if (flags & BF_MATH) h3d_group<true, DIV_RECIP, B3D_W>(p, sd3, k1, acc, prev, x0, iy, iz);
+            else h3d_group<false, DIV_RECIP, B3D_W>(p, sd3, k1, acc, prev, x0, iy, iz);
+        } else if (flags & BF_FAST) {
+            if (flags & BF_MATH) h3d_group<true, DIV_EXACT, B3D_W>(p, sd3, k1, acc, prev, x0, iy, iz);
+            else h3d_group<false, DIV_EXACT, B3D_W>(p, sd3, k1, acc, prev, x0, iy, iz);
+        } else {   // a divisor that needs IEEE division
+            if (flags & BF_MATH) h3d_group<true, DIV_IEEE, B3D_W>(p, sd3, k1, acc, prev, x0, iy, iz);
+            else h3d_group<false, DIV_IEEE, B3D_W>(p, sd3, k1, acc, prev, x0, iy, iz);
         }
     }
 }
 
 template <int DSET>
-__global__ void __launch_bounds__(512, MFD_B3D_MINB) batch_e3d_kernel(const BMember* __restrict__ mem, const BTile* __restrict__ tiles,
-                                                        const int* __restrict__ ntiles) {
+__global__ void __launch_bounds__(512, 2) batch_e3d_kernel(const BMember* __restrict__ mem, const BTile* __restrict__ tiles,
+                                                           const int* __restrict__ ntiles) {
     __shared__ __align__(16) EParams<float, double> sp;
     __shared__ Div3 sd3;
     const int n = *ntiles;
-    int cur = -1;
-    // Tile t of the block's k-th turn: runs of MFD_B3D_CHUNK tiles, the runs dealt out to the
-    // blocks in turn, so t grows with k.
-    for (int k = 0;; ++k) {
-        const int t = ((k / MFD_B3D_CHUNK) * (int)gridDim.x + (int)blockIdx.x) * MFD_B3D_CHUNK + k % MFD_B3D_CHUNK;
-        if (t >= n) break;
-        const BTile tl = tiles[t];
-        const BMember& M = mem[tl.m];
-        if (!b_active(M) || b_other_set<DSET>(M.flags)) continue;   // the same for the whole block
-        const int flags = M.flags;
+    int cur = -1, flags = 0;
+    bool skip = false;
+    BTile nxt = b_tile<MFD_B3D_CHUNK>(tiles, 0, n);   // as in the 2-D kernels
+    for (int k = 0; nxt.m >= 0; ++k) {
+        const BTile tl = nxt;
+        nxt = b_tile<MFD_B3D_CHUNK>(tiles, k + 1, n);
         if (tl.m != cur) {   // the block copies the member's parameters to shared memory
-            __syncthreads();
-            b_stage(&sp, M.ep);
-            if (threadIdx.x == 0 && threadIdx.y == 0) sd3 = M.d3;
-            __syncthreads();
+            const BMember& M = mem[tl.m];
             cur = tl.m;
-        }
-        const EParams<float, double>& p = sp;
-        const Div3& d3 = sd3;
-        int ix, iy, iz;
-        if (!b_cell3(p.L, tl, ix, iy, iz)) continue;
-        if constexpr (DSET == 1) {
-            if (flags & BF_MAT) e3d_cell<float, double, true, DIV_RECIP>(p, d3, ix, iy, iz);
-            else e3d_cell<float, double, false, DIV_RECIP>(p, d3, ix, iy, iz);
-        } else {
-            switch (flags & (BF_MAT | BF_FAST)) {
-                case 0: e3d_cell<float, double, false, DIV_IEEE>(p, d3, ix, iy, iz); break;
-                case BF_MAT: e3d_cell<float, double, true, DIV_IEEE>(p, d3, ix, iy, iz); break;
-                case BF_FAST: e3d_cell<float, double, false, DIV_EXACT>(p, d3, ix, iy, iz); break;
-                default: e3d_cell<float, double, true, DIV_EXACT>(p, d3, ix, iy, iz); break;
+            flags = M.flags;
+            skip = !b_active(M) || b_other_set<DSET>(flags);   // the same for the whole block
+            __syncthreads();
+            if (!skip) {
+                b_stage(&sp, M.ep);
+                if (threadIdx.x == 0 && threadIdx.y == 0) sd3 = M.d3;
             }
+            __syncthreads();
+        }
+        if (skip) continue;
+        const EParams<float, double>& p = sp;
+        int x0, iy, iz;
+        if (!b_group3(p.L, tl, x0, iy, iz)) continue;
+        const bool k1 = flags & BF_K1;
+        if constexpr (DSET == 1) {
+            if (flags & BF_MAT) e3d_group<double, true, DIV_RECIP, B3D_W>(p, sd3, k1, x0, iy, iz);
+            else e3d_group<double, false, DIV_RECIP, B3D_W>(p, sd3, k1, x0, iy, iz);
+        } else if (flags & BF_FAST) {
+            if (flags & BF_MAT) e3d_group<double, true, DIV_EXACT, B3D_W>(p, sd3, k1, x0, iy, iz);
+            else e3d_group<double, false, DIV_EXACT, B3D_W>(p, sd3, k1, x0, iy, iz);
+        } else {   // a divisor that needs IEEE division
+            if (flags & BF_MAT) e3d_group<double, true, DIV_IEEE, B3D_W>(p, sd3, k1, x0, iy, iz);
+            else e3d_group<double, false, DIV_IEEE, B3D_W>(p, sd3, k1, x0, iy, iz);
         }
     }
 }

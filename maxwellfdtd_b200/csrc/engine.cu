@@ -2592,10 +2592,10 @@ struct mfd_batch {
             const bool d3 = e->ndim == 3;
             const int rows = d3 ? e->ny * e->nz : e->nz;   // 3-D: rows y + ny z
             if (d3) {
-                const int ncell = e->nx * rows;
-                for (int l = 0; l < ncell; l += cur_tx * cur_tz) {   // (x, y, z) of the tile's first cell
-                    const int r = l / e->nx;
-                    tiles3.push_back(BTile{mi, l - r * e->nx, r % e->ny, r / e->ny});
+                const int ng = (e->nx + B3D_W - 1) / B3D_W, ngroup = ng * rows;
+                for (int l = 0; l < ngroup; l += cur_tx * cur_tz) {   // (group, y, z) of the tile's first group
+                    const int r = l / ng;
+                    tiles3.push_back(BTile{mi, l - r * ng, r % e->ny, r / e->ny});
                 }
             } else {
                 for (int z = 0; z < rows; z += cur_tz)
