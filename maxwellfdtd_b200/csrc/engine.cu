@@ -834,7 +834,7 @@ class Engine : public HandleBase {
     // ---- resident steps (resident.cuh) -------------------------------------------------
     // Cells up to which the resident steps are the faster way (us per step, separate launches
     // against resident, dispersive model with CPML, one point source and four monitors):
-    //   1-D, any: 3 000 cells 24.3 / 4.5, 60 000 35.0 / 5.0;
+    //   1-D, any: 3 000 cells 24.3 / 4.5 (one cluster: 3.9), 60 000 35.0 / 5.0;
     //   2-D float 301 x 300 22.8 / 6.8, 701 x 700 27.7 / 18.0, 1101 x 1100 36.9 / 34.0;
     //   2-D double 301 x 300 24.6 / 9.7, 901 x 900 35.9 / 31.7, 1101 x 1100 48.4 / 49.2;
     //   3-D float 46 x 45 x 44 36.7 / 9.0, 91 x 90 x 89 54.0 / 43.3 (tolerance mode 83.5 / 36.5);
@@ -882,9 +882,13 @@ class Engine : public HandleBase {
         if (per_sm < 1 || !coop) return;
         ResidentParams<T>& p = res_p;
         p.ncell = (int)N;
-        res_blocks = (int)std::min<long long>((long long)per_sm * sms, (N + RES_MINCELLS - 1) / RES_MINCELLS);
+        // up to one cell per thread of a cluster's blocks: one cluster
+        p.cluster = N > RES_MINCELLS && N <= (long long)RES_CLUSTER * RES_THREADS<T>;
+        res_blocks = p.cluster ? RES_CLUSTER
+                               : (int)std::min<long long>((long long)per_sm * sms, (N + RES_MINCELLS - 1) / RES_MINCELLS);
         p.per = (int)((N + res_blocks - 1) / res_blocks);
         res_blocks = (int)((N + p.per - 1) / p.per);
+        if (res_blocks == 1) p.cluster = false;
         // every round of the block's threads over its cells equally full
         const int rounds = (p.per + RES_THREADS<T> - 1) / RES_THREADS<T>;
         res_threads = (int)round_up((p.per + rounds - 1) / rounds, 32);
@@ -1011,7 +1015,22 @@ class Engine : public HandleBase {
             with_resident_kernel([&](auto k) {
                 long long first = it;
                 void* args[] = {&hp, &ep, &d3, &res_p, &first, &n, &accum, &slot0};
-                MFD_CK(cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)res_blocks), dim3((unsigned)res_threads), args, (size_t)res_smem, st));
+                if (res_p.cluster) {
+                    cudaLaunchConfig_t cfg{};
+                    cfg.gridDim = dim3((unsigned)res_blocks);
+                    cfg.blockDim = dim3((unsigned)res_threads);
+                    cfg.dynamicSmemBytes = (size_t)res_smem;
+                    cfg.stream = st;
+                    cudaLaunchAttribute at{};
+                    at.id = cudaLaunchAttributeClusterDimension;
+                    at.val.clusterDim.x = (unsigned)res_blocks;
+                    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+                    cfg.attrs = &at;
+                    cfg.numAttrs = 1;
+                    MFD_CK(cudaLaunchKernelExC(&cfg, (const void*)k, args));
+                } else {
+                    MFD_CK(cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)res_blocks), dim3((unsigned)res_threads), args, (size_t)res_smem, st));
+                }
             });
         });
         if (!mons_host.empty() && need_ring) ring_used += n;

@@ -20,8 +20,10 @@
 //
 // What bounds it: an empty barrier of 148 blocks takes 1.1 us, then comes the chain L2 load ->
 // arithmetic -> store of about 1 us per half-step for one cell per thread; from about 500 cells
-// per SM on the instructions of the cells.  Measured per step, separate launches / resident:
-// 2 001 cells 1-D double 20.5 / 4.5 us, 201 x 149 float 15.3 / 5.2, 61 x 48 x 55 float 42.7 /
+// per SM on the instructions of the cells.  Up to one cell per thread of eight blocks the grid is
+// one thread-block cluster with the hardware's barrier (2 001 cells: 4.5 us per step with the grid
+// barrier, 3.85 so).  Measured per step, separate launches / resident: 2 001 cells 1-D double
+// 20.5 / 3.85 us, 201 x 149 float 15.3 / 5.2, 61 x 48 x 55 float 42.7 /
 // 12.2, 701 x 513 double 25.2 / 14.9.  The engine's resident_limit says up to which size it is
 // used.
 #pragma once
@@ -37,6 +39,7 @@ namespace mfd {
 template <typename T>
 constexpr int RES_THREADS = sizeof(T) == 4 ? 640 : 512;
 constexpr int RES_MINCELLS = 128;        // cells per block below which no further block is added
+constexpr int RES_CLUSTER = 8;           // blocks of a model that steps as one thread-block cluster
 constexpr int RES_MAXOPS = 32;           // sources (and the TFSF replay) of a resident model
 constexpr unsigned RES_POLLS = 1u << 24; // polls of a barrier before it gives up (seconds)
 constexpr int RES_PRE = 3;               // sources whose next waveform value a thread fetches ahead
@@ -78,6 +81,7 @@ struct ResidentParams {
     int* fault;                  // set when a barrier's wait ran out
     T dt;
     int nmat;
+    bool cluster;                // the grid is one thread-block cluster
     bool k1;                     // every CPML kappa is 1 (the default): no division by it
     // byte offsets of the tables a block copies to dynamic shared memory (-1: left in global
     // memory, too large)
@@ -91,8 +95,14 @@ struct ResidentParams {
 };
 
 // Arrive at and wait for the barrier number k (from 1).  Returns false, in every thread of the
-// block, when the wait ran out.
-__device__ __forceinline__ bool res_barrier(unsigned* bar, unsigned k, int* fault, int* s_ok) {
+// block, when the wait ran out.  A grid of one cluster takes the hardware's cluster barrier (about
+// 0.3 us instead of 1.1 through L2), which every thread reaches: there is no wait to run out.
+__device__ __forceinline__ bool res_barrier(unsigned* bar, unsigned k, int* fault, int* s_ok, bool cluster) {
+    if (cluster) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return true;
+    }
     __syncthreads();
     if (gridDim.x == 1) return true;
     if (threadIdx.x == 0) {
@@ -649,7 +659,7 @@ __global__ void __launch_bounds__(RES_THREADS<T>, 1)
             v.load(hp, acc, ix, iy, iz);
             v.finish(hp, D3, r.k1, acc, it - 1);
         }
-        if (!res_barrier(r.bar, ++bar, r.fault, &s_ok)) return;
+        if (!res_barrier(r.bar, ++bar, r.fault, &s_ok, r.cluster)) return;
         const int cur = (int)((it - 1) & 1);
         for (int l = lo + tid; l < hi; l += nth) {
             int ix = x1, iy = y1, iz = z1;
@@ -701,7 +711,7 @@ __global__ void __launch_bounds__(RES_THREADS<T>, 1)
                 else monitor_point(mp, r.mlist[2 * i], r.mlist[2 * i + 1], it - 1, slot0 + s);
             }
         }
-        if (!res_barrier(r.bar, ++bar, r.fault, &s_ok)) return;
+        if (!res_barrier(r.bar, ++bar, r.fault, &s_ok, r.cluster)) return;
     }
 }
 
