@@ -119,8 +119,8 @@ __device__ __forceinline__ float cdiv<DIV_EXACT, float>(float x, const DivC<floa
 // three divisors and reciprocals and the band common to the three (lob1 = bits(lo) - 1,
 // hib = bits(hi)), so one integer min/max reduction checks all six numerators: a nonzero
 // |x| outside the band, or an unverified divisor, takes the IEEE division in one rarely
-// taken branch.  copysign(q, x) makes zero numerators exact too (q = RN(x/d) has the sign
-// of x since d > 0).
+// taken branch.  The correction is written q = q0 - (q0 d - x) r: for x = +-0 the remainder is +0
+// and q keeps q0's sign, so zero numerators come out as x / d has them.
 struct Div3 {
     float dx, dy, dz, rx, ry, rz;
     unsigned lob1, hib;
@@ -128,16 +128,15 @@ struct Div3 {
 
 __device__ __forceinline__ float qcorr(float x, float d, float r) {
     const float q0 = __fmul_rn(x, r);
-    const float e = __fmaf_rn(-q0, d, x);
-    return copysignf(__fmaf_rn(e, r, q0), x);
+    const float e = __fmaf_rn(q0, d, -x);
+    return __fmaf_rn(-e, r, q0);
 }
 
 // RN(x/d) in double precision for x in the band or zero (see DivC).
 __device__ __forceinline__ double qcorr64(double x, double d, double r) {
     const double q0 = __dmul_rn(x, r);
-    const double q1 = __fma_rn(__fma_rn(-q0, d, x), r, q0);
-    const double q = __fma_rn(__fma_rn(-q1, d, x), r, q1);
-    return __hiloint2double((__double2hiint(q) & 0x7fffffff) | (__double2hiint(x) & 0x80000000), __double2loint(q));
+    const double q1 = __fma_rn(-__fma_rn(q0, d, -x), r, q0);   // signs as in qcorr
+    return __fma_rn(-__fma_rn(q1, d, -x), r, q1);
 }
 
 // The high word of |x| as a band key: 0 for x = 0 only.
