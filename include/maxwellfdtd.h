@@ -365,7 +365,8 @@ MFD_API int mfd_batch_add(mfd_batch* b, mfd_handle* h, int64_t it_last);
 /* Advance every member by up to max_steps steps; members that reach their last step are
  * retired.  n_active receives the number of members still running. */
 MFD_API int mfd_batch_run(mfd_batch* b, int64_t max_steps, int32_t* n_active);
-/* Tile shape of the persistent launches (tile_x a multiple of 32, tile_x*tile_z <= 512;
+/* Tile shape of the persistent launches in threads (tile_x a multiple of 32, tile_x*tile_z <=
+ * 512; a thread takes four cells of a row of a 2-D member, two of a 3-D member;
  * 0, 0 = autotune: the first graph replays try candidate shapes and keep the cheapest per
  * cell-update -- results do not depend on the shape) and steps per graph (0 = keep). */
 MFD_API int mfd_batch_config(mfd_batch* b, int32_t tile_x, int32_t tile_z, int32_t graph_steps);

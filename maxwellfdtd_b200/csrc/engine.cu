@@ -863,7 +863,8 @@ class Engine : public HandleBase {
     // Which models step by the resident kernel, and its per-block lists of source and monitor
     // points.  Not: models of a server (overlap = false: many run at once, and a cooperative
     // launch waits until all of its blocks fit), TFSF recording, plasma (its transcendental
-    // code, and compute-bound), more than three poles, divisors that failed the check, CPML layers that overlap, more than RES_MAXOPS sources.
+    // code, and compute-bound), more than three poles, divisors that failed the check, CPML
+    // layers that overlap, more than RES_MAXOPS sources.
     void init_resident(const mfd_desc* d) {
         if (!std::is_same<R, double>::value || !overlap || record || any_plasma || N > resident_limit(ndim)) return;
         if (!recip && !fastdiv) return;
@@ -1747,11 +1748,9 @@ class Engine : public HandleBase {
         e3d_f32_kernel<R, MAT, FAST><<<grd, blk, 0, st>>>(p, d3, zc3);
     }
 
-    // Calls f with the division mode of the model's kernels as a compile-time constant:
-    // DIV_RECIP in the tolerance mode, else DIV_EXACT when every divisor passed the device
-    // check, else DIV_IEEE.
+    // As with_div, with DIV_EXACT1 (no division by kappa) where every kappa is 1.
     template <typename F_>
-    void with_div1(F_&& f) {   // DIV_EXACT1 when every kappa is 1
+    void with_div1(F_&& f) {
         if constexpr (sizeof(T) == 4) {
             if (!recip && fastdiv && kappa_one) {
                 f(std::integral_constant<int, DIV_EXACT1>{});
@@ -1760,6 +1759,9 @@ class Engine : public HandleBase {
         }
         with_div(f);
     }
+    // Calls f with the division mode of the model's kernels as a compile-time constant:
+    // DIV_RECIP in the tolerance mode, else DIV_EXACT when every divisor passed the device
+    // check, else DIV_IEEE.
     template <typename F_>
     void with_div(F_&& f) {
         if (recip) f(std::integral_constant<int, DIV_RECIP>{});
@@ -2620,8 +2622,8 @@ struct mfd_batch {
                 for (int z = 0; z < rows; z += cur_tz)
                     for (int x = 0; x < e->nx; x += 4 * cur_tx) tiles.push_back(BTile{mi, x, z, 0});
             }
-            if (!(m.flags & BF_RESP))   // else the E update takes the response
             for (int g : e->response_mats) {
+                if (m.flags & BF_RESP) break;   // the E update takes the response
                 const MatDev<float, double>& md = e->mats_host[g - 1];
                 const int y0 = d3 ? md.by0 : 0, y1 = d3 ? md.by0 + md.bny : 1;
                 for (int z = md.bz0; z < md.bz0 + md.bnz; ++z)

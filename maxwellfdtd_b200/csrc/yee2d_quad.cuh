@@ -16,7 +16,7 @@
 // one cell per thread and the material kernel, 37.1 now (41.6 with the psi loads after the first
 // stores; the batched kernels, which hold their parameters in shared memory, spill with them ahead:
 // 262 -> 287 us, so they keep them behind); 32 batched
-// models of 128-1024 cells a side, exact mode 277 us, 254 now (latency: 45 % of the warps active).
+// models of 128-1024 cells a side, exact mode 277 us, 250 now (latency: 45 % of the warps active).
 #pragma once
 
 #include "yee.cuh"
