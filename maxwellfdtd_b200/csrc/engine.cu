@@ -419,12 +419,16 @@ class Engine : public HandleBase {
     // planes per block of the material-row E launch: one (more, shorter-lived blocks beside
     // the staged kernel's; 256^3 plasmonics: E 0.193 ms per update against 0.198 at 4)
     int zc_mat = 1;
-    // The y- and z-layer cells of the single-precision split updates go through the staged
-    // kernels (LAY 1 / 2) instead of the one-cell-per-thread slab kernels: in the tolerance
-    // mode, for the H update (256^3 plasmonics: 43.5 against 42.5 Gcell/s with both updates
-    // layered; the exact mode's layer code needs 80 registers and measured slower, 38.0
-    // against 40.2).
-    bool lay_H = true, lay_E = true;
+    // The y- and z-layer cells of the single-precision split updates in the tolerance mode go
+    // through the staged kernels (LAY 1 / 2, one launch per side) instead of the
+    // one-cell-per-thread slab kernels (one launch) from LAYERED_MIN cells on: below, the
+    // short marches of eight layer launches a step cost more than the slab kernels' extra
+    // instructions.  us per step, layered / slab (10-cell CPML, dispersive medium): 101 x 100 x
+    // 99 90 / 51, 129 x 128 x 127 129 / 99, 161 x 160 x 159 172 / 157, 177 x 176 x 175 191 / 182,
+    // 201 x 200 x 199 255.7 / 255.3 (TFSF in vacuum 226 / 233), 257 x 256 x 255 459 / 486.  The exact
+    // mode's layer code needs 80 registers and measured slower at 256^3 (38.0 against 40.2 Gcell/s).
+    static constexpr long long LAYERED_MIN = 6500000;
+    bool layered = false;
     // Planes per block of a z-layer launch of n planes: the whole layer in one march up to 16
     // planes, else even chunks of at most 12.  At 256^3 plasmonics (13-plane layers, side
     // streams at the highest priority): 13 gave 44.64-44.65 against 44.31-44.32 for chunks of
@@ -837,7 +841,7 @@ class Engine : public HandleBase {
     //   1-D, any: 3 000 cells 24.3 / 4.5 (one cluster: 3.9), 60 000 35.0 / 5.0;
     //   2-D float 301 x 300 22.8 / 6.8, 701 x 700 27.7 / 18.0, 1101 x 1100 36.9 / 34.0;
     //   2-D double 301 x 300 24.6 / 9.7, 901 x 900 35.9 / 31.7, 1101 x 1100 48.4 / 49.2;
-    //   3-D float 46 x 45 x 44 36.7 / 9.0, 91 x 90 x 89 54.0 / 43.3 (tolerance mode 83.5 / 36.5);
+    //   3-D float 46 x 45 x 44 36.7 / 9.0, 91 x 90 x 89 54.0 / 43.3 (tolerance mode 43 / 36.5);
     //   3-D double 46 x 45 x 44 37.5 / 12.7, 91 x 90 x 89 69.8 / 57.4, 100^3 82 / 102.
     static long long resident_limit(int nd) { return nd == 3 ? 750000 : 1000000; }
 
@@ -1076,14 +1080,14 @@ class Engine : public HandleBase {
         if (xl > xr || yl > yr || zl > zr) return;
         if (const char* a = std::getenv("MFD_CORE_ASYNC")) core_async = std::atoi(a) != 0;
         if (const char* z = std::getenv("MFD_ASYNC_ZC")) async_zc = std::max(1, std::atoi(z));
-        // In the tolerance mode the y layers' rows go through the staged kernel in tiles of
-        // AS_TY rows.  Each y-layer launch is widened to whole tiles: the rows it gains are
+        layered = sizeof(T) == 4 && recip && core_async && N >= LAYERED_MIN;
+        // Layered, the y layers' rows go through the staged kernel in tiles of AS_TY rows.  Each y-layer launch is widened to whole tiles: the rows it gains are
         // core rows, which that kernel updates as the core launch would (no y face there), so
         // no layer tile runs with idle rows and the core box starts on a tile (256^3
         // plasmonics: 13-row layers become 16-row launches, the core 224 rows; 44.77-44.82
-        // against 44.59-44.63 Gcell/s on one box).  The exact mode keeps the layer bounds:
-        // its slab kernels update the rows outside the core box one cell per thread.
-        if (sizeof(T) == 4 && recip && core_async) {
+        // against 44.59-44.63 Gcell/s on one box).  Otherwise the layer bounds stay: the slab
+        // kernels update the rows outside the core box one cell per thread.
+        if (layered) {
             const int yl_a = (yl + AS_TY - 1) / AS_TY * AS_TY;
             const int yr_a = ny - (ny - yr + AS_TY - 1) / AS_TY * AS_TY;
             if (yl_a < yr_a) { yl = yl_a; yr = yr_a; }
@@ -1572,7 +1576,7 @@ class Engine : public HandleBase {
         kcount = 0;
         const int zn = sbox.zr - sbox.zl;
         const bool core = sbox.yr > sbox.yl && zn > 0;
-        const bool lay = sizeof(T) == 4 && core_async && lay_H && recip && core && slab_rows;
+        const bool lay = layered && core && slab_rows;
         const bool ov = st_side && slab_rows && core;
         if (ov) fork(lay);
         if constexpr (sizeof(T) == 4)
@@ -1684,7 +1688,7 @@ class Engine : public HandleBase {
                 kcount++;
             }
         }
-        const bool lay = sizeof(T) == 4 && core_async && lay_E && recip && core && slab_rows;
+        const bool lay = layered && core && slab_rows;
         if constexpr (sizeof(T) == 4) {
             if (lay) {
                 if (MAT && mat_in_layers) launch_E_layers<true, FAST>(p, ov ? st_side : st, ov ? st_side2 : st);

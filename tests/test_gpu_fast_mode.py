@@ -251,3 +251,23 @@ def test_fast_mode_thick_z_layers(oracle_lib, gpu_lib):
     ref = C.run_all(model, oracle_lib, np.float32, mons)
     got = C.run_all(model, gpu_lib, np.float32, mons, mode="fast")
     _check(ref, got, np.float32, lambda: C.run_all(model, oracle_lib, np.float64, mons))
+
+
+@pytest.mark.parametrize("pml_on", ["all", "z"])
+@pytest.mark.parametrize("nz", [166, 171])
+def test_fast_mode_layer_launches(nz, pml_on, gpu_lib):
+    """Grids of 6.47 and 6.67 million cells, on both sides of the size from which the tolerance
+    mode's y and z layers go through the staged kernels, with a Drude+Lorentz ball that reaches
+    into the y layer: the tolerance mode against the exact mode, which the oracle pins."""
+    g = C.grid3((205, 190, nz))
+    z0 = g.z[0] + 600e-9   # 4 cells from the z layer, which the wave enters
+    src = M.SoftSource(geometry=C._plane(3, z0), waveform=C._src_wave(3, 2e8), component="Ex")
+    dt = 0.5 / C.C0 / np.sqrt(3 / (50e-9) ** 2)
+    ball = C._ball(3, 500e-9, (0.0, -4.3e-6, z0))
+    m = M.Material(geometry=ball, eps=3.0, chi=[M.DrudeSusceptibility(wp=1.37e16, gamma=1.07e14),
+                                                M.LorentzSusceptibility(deps=1.1, w0=4.2e15, delta=5e14)])
+    pml = 400e-9 if pml_on == "all" else (0, 0, 0, 0, 400e-9, 400e-9)
+    model = M.Model(g, src, tmax=(30 - 0.5) * dt, pml=pml, material=[m])
+    ref = C.run_all(model, gpu_lib, np.float32)
+    got = C.run_all(model, gpu_lib, np.float32, mode="fast")
+    _check(ref, got, np.float32)
