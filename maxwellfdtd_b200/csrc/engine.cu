@@ -452,6 +452,7 @@ class Engine : public HandleBase {
 
     // Small models: many steps in one cooperative launch (resident.cuh)
     bool resident = false;
+    bool res_hpts = false;      // some source writes H
     ResidentParams<T> res_p{};
     int res_blocks = 0, res_threads = 0, res_smem = 0;
     int* d_resfault = nullptr;
@@ -850,8 +851,12 @@ class Engine : public HandleBase {
         if constexpr (std::is_same<R, double>::value) {
             auto pick = [&](auto fs, auto dm) {
                 constexpr int FS = decltype(fs)::value, D = decltype(dm)::value;
-                if (any_geom) f(resident_kernel<T, R, FS, true, D>);
-                else f(resident_kernel<T, R, FS, false, D>);
+                auto mat = [&](auto hp) {
+                    if (any_geom) f(resident_kernel<T, R, FS, true, D, decltype(hp)::value>);
+                    else f(resident_kernel<T, R, FS, false, D, decltype(hp)::value>);
+                };
+                if (res_hpts) mat(std::true_type{});
+                else mat(std::false_type{});
             };
             auto dims = [&](auto dm) {
                 if (ndim == 1) pick(std::integral_constant<int, 1>{}, dm);
@@ -878,8 +883,10 @@ class Engine : public HandleBase {
             if (mats_host[g - 1].nq > 3) return;
         for (int f = 0; f < 6; f += 2)   // a cell in both layers of an axis (they overlap)
             if (lay[f].nb && lay[f + 1].nb && lay[f].ib > lay[f + 1].ib - 1) return;
-        const int nops = (int)srcs.size() + (tfsf ? 1 : 0);
-        if (nops > RES_MAXOPS) return;
+        if ((int)srcs.size() + (tfsf ? 1 : 0) > RES_MAXOPS) return;
+        const int nops = (int)srcs.size() + (tfsf ? 2 : 0);   // the TFSF replay: on E and D, and on H
+        res_hpts = tfsf;
+        for (const Src& S : srcs) res_hpts = res_hpts || S.comp <= MFD_HZ;
         int per_sm = 0, sms = 0, coop = 0;
         with_resident_kernel([&](auto k) { MFD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, RES_THREADS<T>, 0)); });
         MFD_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -946,30 +953,34 @@ class Engine : public HandleBase {
             all.insert(all.end(), ent.begin(), ent.end());
         };
         std::vector<ResOp<T>> ops;
-        for (size_t i = 0; i <= srcs.size(); ++i) {
-            if (tfsf && (int)i == tfsf_order) {
-                add_list(2, [&](auto&& emit) {
-                    for (int k = 0; k < tfsf_p.n; ++k) {
-                        const RectStmt& q = tfsf_p.s[k];
-                        int local = 0;
-                        for (int z = q.z0; z <= q.z1; ++z)
-                            for (int y = q.y0; y <= q.y1; ++y)
-                                for (int x = q.x0; x <= q.x1; ++x, ++local) emit((long long)x + (long long)nx * (y + (long long)ny * z), k, local);
-                    }
-                });
-                ResOp<T> o{};
-                o.tfsf = 1;
-                ops.push_back(o);
+        for (int onh = 0; onh < 2; ++onh) {   // sources on E and D, then those on H
+            for (size_t i = 0; i <= srcs.size(); ++i) {
+                if (tfsf && (int)i == tfsf_order) {
+                    add_list(2, [&](auto&& emit) {
+                        for (int k = 0; k < tfsf_p.n; ++k) {
+                            const RectStmt& q = tfsf_p.s[k];
+                            if ((q.comp <= MFD_HZ) != (onh != 0)) continue;
+                            int local = 0;
+                            for (int z = q.z0; z <= q.z1; ++z)
+                                for (int y = q.y0; y <= q.y1; ++y)
+                                    for (int x = q.x0; x <= q.x1; ++x, ++local) emit((long long)x + (long long)nx * (y + (long long)ny * z), k, local);
+                        }
+                    });
+                    ResOp<T> o{};
+                    o.tfsf = 1;
+                    ops.push_back(o);
+                }
+                if (i < srcs.size() && (srcs[i].comp <= MFD_HZ) == (onh != 0)) {
+                    const int64_t* cells = d->srcs[i].cells;
+                    const Src& S = srcs[i];
+                    add_list(1, [&](auto&& emit) { for (long long j = 0; j < S.npts; ++j) emit(cells[j], (int)j, 0); });
+                    ResOp<T> o{};
+                    o.kind = S.kind; o.coeff = S.coeff; o.F = F[S.comp]; o.cells = S.cells; o.wave = S.wave; o.amp = S.amp;
+                    o.gt = S.gt; o.npts = S.npts;
+                    ops.push_back(o);
+                }
             }
-            if (i < srcs.size()) {
-                const int64_t* cells = d->srcs[i].cells;
-                const Src& S = srcs[i];
-                add_list(1, [&](auto&& emit) { for (long long j = 0; j < S.npts; ++j) emit(cells[j], (int)j, 0); });
-                ResOp<T> o{};
-                o.kind = S.kind; o.coeff = S.coeff; o.F = F[S.comp]; o.cells = S.cells; o.wave = S.wave; o.amp = S.amp;
-                o.gt = S.gt; o.npts = S.npts;
-                ops.push_back(o);
-            }
+            if (!onh) p.nops_e = (int)ops.size();
         }
         p.nops = (int)ops.size();
         p.nmon = mon_p.nmon;

@@ -6,11 +6,16 @@
 // owns a contiguous run of cells (x-fastest order) and one thread always updates the same cell,
 // so per step the blocks meet only twice, at a grid barrier after the H update and at one after
 // the E update:
-//   H update (+ running sums and guard of the step before)        | barrier
-//   E update, material response, sources, monitor gather           | barrier
-// The sources and the monitors of a step need no barrier of the grid because a block applies
-// the source points, TFSF points and monitor points that lie in its own cells (lists made on
-// the host per block), in the order of the model's sources, after its own E update.
+//   H update (+ running sums and guard of the step before)              | barrier
+//   E update, material response, source points on E and D, monitor points | barrier
+//   source points on H (and the monitor points of a block that has such)
+// A block applies the source points, TFSF points and monitor points that lie in its own cells
+// (lists made on the host per block), in the order of the model's sources.  Points on E and D follow
+// the block's own E update: between the two barriers no other block reads its E or D.  Points on H
+// have to wait for the second barrier: until then other blocks may still read that H for their E
+// update.  After it, up to the next barrier, H is read by its own block only, so they go before the
+// block's next H update, and the block's monitor points, which read H, go after them.  Order between
+// sources matters within one component only, which the split keeps.
 //
 // The arithmetic is the single-launch kernels' (h1d_kernel ... e3d_cell, material_cell_n, the
 // point-source expression, tfsf_point), operation for operation, so results are bit-identical.
@@ -40,12 +45,13 @@ template <typename T>
 constexpr int RES_THREADS = sizeof(T) == 4 ? 640 : 512;
 constexpr int RES_MINCELLS = 128;        // cells per block below which no further block is added
 constexpr int RES_CLUSTER = 8;           // blocks of a model that steps as one thread-block cluster
-constexpr int RES_MAXOPS = 32;           // sources (and the TFSF replay) of a resident model
+constexpr int RES_MAXOPS = 32;           // sources (and the TFSF replay, one) of a resident model
 constexpr unsigned RES_POLLS = 1u << 24; // polls of a barrier before it gives up (seconds)
 constexpr int RES_PRE = 3;               // sources whose next waveform value a thread fetches ahead
 
-// One source of the model in its tuple order: the points of block b are entries
-// list[off[b]] .. list[off[b + 1] - 1] (a point index, or for TFSF the pair (statement, local)).
+// One source of the model (the TFSF replay twice: its statements on E and D and those on H), those
+// on E and D first, then those on H, each group in the model's tuple order: the points of block b are
+// entries list[off[b]] .. list[off[b + 1] - 1] (a point index, or for TFSF the pair (statement, local)).
 template <typename T>
 struct ResOp {
     int tfsf, kind;
@@ -92,6 +98,7 @@ struct ResidentParams {
     int o_mon;                   // monitor descriptors
     int o_ops;                   // the sources
     int o_pts, npts_cap;         // the block's source and monitor points (ResPoint)
+    int nops_e;                  // sources on E and D: the first of the nops
 };
 
 // Arrive at and wait for the barrier number k (from 1).  Returns false, in every thread of the
@@ -516,15 +523,48 @@ struct ResE {
     }
 };
 
+// A source's points a .. b - 1 of this block at step it0 (0-based), as the kernel below applies them;
+// pts: those points in shared memory, or null.  pre: w0 is the waveform value of the thread's first.
+template <typename T>
+__device__ __forceinline__ void res_source(const ResOp<T>& op, const RectParams<T>& rp, const ResPoint* pts, int a, int b, long long it0,
+                                           bool pre, double w0) {
+    for (int i = a + (int)threadIdx.x; i < b; i += blockDim.x) {
+        if (op.tfsf) {
+            if (pts) tfsf_point(rp, pts[i - a].m, pts[i - a].j, it0);
+            else tfsf_point(rp, op.list[2 * i], op.list[2 * i + 1], it0);
+            continue;
+        }
+        const int j = pts ? pts[i - a].j : op.list[i];
+        const long long c = pts ? pts[i - a].c : op.cells[j];
+        double w = pre && pts && i == a + (int)threadIdx.x ? w0 : op.wave ? op.wave[it0 * op.npts + j] : op.gt[it0];
+        if (!op.wave) w = (pts ? pts[i - a].amp : op.amp[j]) * w;
+        if (op.kind == MFD_SRC_SOFT) op.F[c] = (T)((double)op.F[c] + (double)op.coeff * w);
+        else op.F[c] = (T)w;
+    }
+}
+
+// The block's monitor points a .. b - 1; pts as above.
+template <typename T>
+__device__ __forceinline__ void res_monitors(const MonParams<T>& mp, const int* list, const ResPoint* pts, int a, int b, long long it0, int slot) {
+    for (int i = a + (int)threadIdx.x; i < b; i += blockDim.x) {
+        if (pts) monitor_store(mp, mp.mons[pts[i - a].m], pts[i - a].j, pts[i - a].c, it0, slot);
+        else monitor_point(mp, list[2 * i], list[2 * i + 1], it0, slot);
+    }
+}
+
 // FS: 1, 2, 3 (the model's dimension) or FSET_EY2.  MAT: the model has a material map.
-template <typename T, typename R, int FS, bool MAT, int FAST>
+// HPTS: some source writes H.  Models without such take the step's plain order, in code of its own:
+// sharing the two-part form with them cost 0.8 % of a step of 2001 cells (double, 3.68 -> 3.71 us) and
+// 3.6 % of one of 701 x 513 (double, second field set, 15.7 -> 16.3 us), whatever the loop's form.
+template <typename T, typename R, int FS, bool MAT, int FAST, bool HPTS>
 __global__ void __launch_bounds__(RES_THREADS<T>, 1)
     resident_kernel(const __grid_constant__ HParams<T> hp0, const __grid_constant__ EParams<T, R> ep0, const Div3 D3,
                     const __grid_constant__ ResidentParams<T> r, const long long it_first, const int nsteps, const int accum,
                     const int slot0) {
     extern __shared__ __align__(16) char sm[];
     __shared__ int s_ok;
-    __shared__ int s_op[RES_MAXOPS + 1][2];   // this block's entries of each source; the last row: its monitor points
+    constexpr int MON_ROW = HPTS ? RES_MAXOPS + 1 : RES_MAXOPS;
+    __shared__ int s_op[MON_ROW + 1][2];   // this block's entries of each source; the last row: its monitor points
     const int tid = threadIdx.x, nth = blockDim.x;
     const int nx = hp0.L.nx, ny = hp0.L.ny, px = hp0.L.px, sz = hp0.L.sz;
     const int lo = blockIdx.x * r.per, hi = min(lo + r.per, r.ncell);
@@ -591,12 +631,16 @@ __global__ void __launch_bounds__(RES_THREADS<T>, 1)
     }
     if (tid == 0) {
         s_ok = 1;
-        s_op[RES_MAXOPS][0] = r.nmon ? r.moff[blockIdx.x] : 0;
-        s_op[RES_MAXOPS][1] = r.nmon ? r.moff[blockIdx.x + 1] : 0;
+        s_op[MON_ROW][0] = r.nmon ? r.moff[blockIdx.x] : 0;
+        s_op[MON_ROW][1] = r.nmon ? r.moff[blockIdx.x + 1] : 0;
     }
     if (tid < r.nops) {
         s_op[tid][0] = r.ops[tid].off[blockIdx.x];
         s_op[tid][1] = r.ops[tid].off[blockIdx.x + 1];
+    }
+    if (HPTS && tid == 0 && r.nops > RES_MAXOPS) {   // a block has at least 32 threads
+        s_op[RES_MAXOPS][0] = r.ops[RES_MAXOPS].off[blockIdx.x];
+        s_op[RES_MAXOPS][1] = r.ops[RES_MAXOPS].off[blockIdx.x + 1];
     }
     __syncthreads();
     // The block's points, source by source and then the monitors', as far as they fit: point k of
@@ -606,7 +650,7 @@ __global__ void __launch_bounds__(RES_THREADS<T>, 1)
         int k0 = 0;
         for (int o = 0; o <= r.nops; ++o) {
             const bool mon = o == r.nops;
-            const int a = s_op[mon ? RES_MAXOPS : o][0], b = s_op[mon ? RES_MAXOPS : o][1];
+            const int a = s_op[mon ? MON_ROW : o][0], b = s_op[mon ? MON_ROW : o][1];
             for (int i = a + tid; i < b && k0 + i - a < r.npts_cap; i += nth) {
                 ResPoint q{0, 0, 0, 0, 0.0};
                 if (mon) {
@@ -630,8 +674,11 @@ __global__ void __launch_bounds__(RES_THREADS<T>, 1)
     const bool fit = [&] {   // every point of the block is in pts
         int n = 0;
         for (int o = 0; o < r.nops; ++o) n += s_op[o][1] - s_op[o][0];
-        return n + s_op[RES_MAXOPS][1] - s_op[RES_MAXOPS][0] <= r.npts_cap;
+        return n + s_op[MON_ROW][1] - s_op[MON_ROW][0] <= r.npts_cap;
     }();
+    bool tail = false;   // the block has points that write H
+    if constexpr (HPTS)
+        for (int o = r.nops_e; o < r.nops; ++o) tail = tail || s_op[o][1] > s_op[o][0];
     int x1, y1, z1;   // the thread's first cell
     decode(min(lo + tid, hi - 1), x1, y1, z1);
     unsigned bar = 0;
@@ -668,6 +715,31 @@ __global__ void __launch_bounds__(RES_THREADS<T>, 1)
             v.load(ep, ix, iy, iz);
             v.finish(ep, D3, r.k1, ix, iy, iz, cur, r.dt);
         }
+        if constexpr (HPTS) {
+            int o = 0, k0 = 0;
+#pragma unroll 1
+            for (bool late = false;; late = true) {   // late: after the second barrier
+                for (const int end = late ? r.nops : r.nops_e; o < end; ++o) {
+                    const int a = s_op[o][0], b = s_op[o][1];
+                    if (a == b) continue;   // the same for the whole block
+                    __syncthreads();
+                    res_source(ops[o], *rp, fit ? pts + k0 : nullptr, a, b, it - 1, o < RES_PRE, o == 0 ? wpre[0] : o == 1 ? wpre[1] : wpre[2]);
+                    k0 += b - a;
+                }
+                const int ma = s_op[MON_ROW][0], mb = s_op[MON_ROW][1];
+                if (mb > ma && late == tail) {
+                    __syncthreads();
+                    res_monitors(mp, r.mlist, fit ? pts + k0 : nullptr, ma, mb, it - 1, slot0 + s);
+                }
+                if (late) {
+                    __syncthreads();   // the next H update changes what these points wrote and read
+                    break;
+                }
+                if (!res_barrier(r.bar, ++bar, r.fault, &s_ok, r.cluster)) return;
+                if (!tail) break;
+            }
+            continue;
+        }
         // the block's own source points, source by source, then its monitor points
         int k0 = 0;
         for (int o = 0; o < r.nops; ++o) {
@@ -700,7 +772,7 @@ __global__ void __launch_bounds__(RES_THREADS<T>, 1)
             }
             k0 += b - a;
         }
-        const int ma = s_op[RES_MAXOPS][0], mb = s_op[RES_MAXOPS][1];
+        const int ma = s_op[MON_ROW][0], mb = s_op[MON_ROW][1];
         if (mb > ma) {
             __syncthreads();
             for (int i = ma + tid; i < mb; i += nth) {
