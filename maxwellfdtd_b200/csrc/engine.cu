@@ -502,15 +502,23 @@ class Engine : public HandleBase {
     char* chunk = nullptr;
     size_t chunk_left = 0, chunk_next = 256u << 10;
 
-    void* raw_alloc(size_t n) {
+    // n bytes, zeroed; null, with the reason in e, when the device has none.
+    void* try_alloc(size_t n, cudaError_t* e = nullptr) {
         void* p = nullptr;
-        cudaError_t e = cudaMallocAsync(&p, n, st);
-        if (e != cudaSuccess) {
+        const cudaError_t rc = cudaMallocAsync(&p, n, st);
+        if (e) *e = rc;
+        if (rc != cudaSuccess) {
             cudaGetLastError();
-            throw Error(MFD_ERR_OOM, "device allocation of " + std::to_string(n) + " bytes failed: " + cudaGetErrorString(e));
+            return nullptr;
         }
         allocs.push_back(p);
         MFD_CK(cudaMemsetAsync(p, 0, n, st));
+        return p;
+    }
+    void* raw_alloc(size_t n) {
+        cudaError_t e;
+        void* p = try_alloc(n, &e);
+        if (!p) throw Error(MFD_ERR_OOM, "device allocation of " + std::to_string(n) + " bytes failed: " + cudaGetErrorString(e));
         return p;
     }
 
@@ -2185,22 +2193,28 @@ class Engine : public HandleBase {
     // rows of 244 bytes (nx = 61) came at 5.8 GB/s and rows of 200-500 bytes at 16 GB/s, where
     // rows of 924 bytes reach 44.  Shorter rows are therefore packed on the device (a few us)
     // and copied densely, PACK_BYTES at a time (61 x 48 x 55: 11 arrays and 24 traces 1.28 -> 0.67 ms;
-    // 32 models of 48-128 cells a side: 41 -> 34 ms).  noalloc: the
-    // caller's read may not take device memory.
+    // 32 models of 48-128 cells a side: 41 -> 34 ms).  A device without
+    // memory for the buffer still has the strided copy.  noalloc: the caller's read may not take
+    // device memory.
     static constexpr size_t PACK_ROW = 1024, PACK_BYTES = 8u << 20;
     unsigned char* pack_buf = nullptr;
 
     template <typename U>
-    void copy_packed(const void* dsrc, void* hdst) {
+    bool copy_packed(const void* dsrc, void* hdst) {   // false: no memory for the buffer, nothing copied
         const size_t cap = std::min((size_t)N * sizeof(double), PACK_BYTES);   // holds a row of any element type
         const long long rows = (long long)ny * nz, per = (long long)(cap / sizeof(U)) / nx;
-        if (!pack_buf) pack_buf = dalloc<unsigned char>(cap, false);
+        if (!pack_buf) {
+            pack_buf = (unsigned char*)try_alloc(cap);
+            if (!pack_buf) return false;
+            bytes += (int64_t)cap;
+        }
         for (long long r = 0; r < rows; r += per) {
             const long long n = std::min(per, rows - r) * nx;
             pack_rows_kernel<U><<<(unsigned)std::min((n + 255) / 256, 148ll * 8), 256, 0, st>>>((const U*)dsrc, (U*)pack_buf, nx, px, r, n);
             MFD_CK(cudaGetLastError());
             MFD_CK(cudaMemcpyAsync((U*)hdst + r * nx, pack_buf, (size_t)n * sizeof(U), cudaMemcpyDeviceToHost, st));
         }
+        return true;
     }
 
     void copy_out(const void* dsrc, void* hdst, size_t esize, bool noalloc = false) {
@@ -2210,15 +2224,12 @@ class Engine : public HandleBase {
             bounded_sync(st);
             return;
         }
-        if (!noalloc && (size_t)nx * esize < PACK_ROW) {
-            if (esize == 1) copy_packed<uint8_t>(dsrc, hdst);
-            else if (esize == 4) copy_packed<uint32_t>(dsrc, hdst);
-            else copy_packed<uint64_t>(dsrc, hdst);
-            bounded_sync(st);
-            return;
-        }
-        MFD_CK(cudaMemcpy2DAsync(hdst, (size_t)nx * esize, dsrc, (size_t)px * esize, (size_t)nx * esize, (size_t)ny * nz,
-                                 cudaMemcpyDeviceToHost, st));
+        const bool packed = !noalloc && (size_t)nx * esize < PACK_ROW &&
+                            (esize == 1 ? copy_packed<uint8_t>(dsrc, hdst) : esize == 4 ? copy_packed<uint32_t>(dsrc, hdst)
+                                                                                       : copy_packed<uint64_t>(dsrc, hdst));
+        if (!packed)
+            MFD_CK(cudaMemcpy2DAsync(hdst, (size_t)nx * esize, dsrc, (size_t)px * esize, (size_t)nx * esize, (size_t)ny * nz,
+                                     cudaMemcpyDeviceToHost, st));
         bounded_sync(st);
     }
 
