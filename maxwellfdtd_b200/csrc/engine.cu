@@ -451,8 +451,10 @@ class Engine : public HandleBase {
     int kcount = 1;             // kernels issued by the current launch() call
 
     // Small models: many steps in one cooperative launch (resident.cuh)
-    bool resident = false;
+    bool resident = false;      // the model steps so, unless profiled or stepped by a batch
+    bool res_ready = false;     // its lists and tables are on the device: from its first such run on
     bool res_hpts = false;      // some source writes H
+    std::vector<std::vector<int>> res_cells;   // until then: dense cells of each source, then of each monitor
     ResidentParams<T> res_p{};
     int res_blocks = 0, res_threads = 0, res_smem = 0;
     int* d_resfault = nullptr;
@@ -838,7 +840,11 @@ class Engine : public HandleBase {
         h_flags_v.assign((size_t)nt, 0);
         h_flags = h_flags_v.data();
         init_split();
-        init_resident(d);
+        resident = resident_model();
+        if (resident) {
+            for (int i = 0; i < d->nsrc; ++i) res_cells.emplace_back(d->srcs[i].cells, d->srcs[i].cells + d->srcs[i].npts);
+            for (int m = 0; m < d->nmon; ++m) res_cells.emplace_back(d->mons[m].cells, d->mons[m].cells + d->mons[m].npts);
+        }
         mon_apart = overlap && !resident && monitors_apart_from_sources(d);
         MFD_CK(cudaStreamSynchronize(st));
         held.clear();
@@ -877,21 +883,25 @@ class Engine : public HandleBase {
         }
     }
 
-    // Which models step by the resident kernel, and its per-block lists of source and monitor
-    // points.  Not: models of a server (overlap = false: many run at once, and a cooperative
-    // launch waits until all of its blocks fit), TFSF recording, plasma (its transcendental
-    // code, and compute-bound), more than three poles, divisors that failed the check, CPML
-    // layers that overlap, more than RES_MAXOPS sources.
-    void init_resident(const mfd_desc* d) {
-        if (!std::is_same<R, double>::value || !overlap || record || any_plasma || N > resident_limit(ndim)) return;
-        if (!recip && !fastdiv) return;
+    // Which models step by the resident kernel.  Not: models of a server (overlap = false: many run at
+    // once, and a cooperative launch waits until all of its blocks fit), TFSF recording, plasma (its
+    // transcendental code, and compute-bound), more than three poles, divisors that failed the check,
+    // CPML layers that overlap, more than RES_MAXOPS sources.
+    bool resident_model() const {
+        if (!std::is_same<R, double>::value || !overlap || record || any_plasma || N > resident_limit(ndim)) return false;
+        if (!recip && !fastdiv) return false;
         // an explicit choice of the 3-D kernels keeps them
-        if (ndim == 3 && (std::getenv("MFD_KERNEL3D") || std::getenv("MFD_CORE_ASYNC"))) return;
+        if (ndim == 3 && (std::getenv("MFD_KERNEL3D") || std::getenv("MFD_CORE_ASYNC"))) return false;
         for (int g : response_mats)
-            if (mats_host[g - 1].nq > 3) return;
+            if (mats_host[g - 1].nq > 3) return false;
         for (int f = 0; f < 6; f += 2)   // a cell in both layers of an axis (they overlap)
-            if (lay[f].nb && lay[f + 1].nb && lay[f].ib > lay[f + 1].ib - 1) return;
-        if ((int)srcs.size() + (tfsf ? 1 : 0) > RES_MAXOPS) return;
+            if (lay[f].nb && lay[f + 1].nb && lay[f].ib > lay[f + 1].ib - 1) return false;
+        return (int)srcs.size() + (tfsf ? 1 : 0) <= RES_MAXOPS;
+    }
+
+    // The launch shape and the per-block lists of source and monitor points, at the first run that steps
+    // so: a model that a batch steps needs neither.  False: the grid would not be resident at once.
+    bool init_resident() {
         const int nops = (int)srcs.size() + (tfsf ? 2 : 0);   // the TFSF replay: on E and D, and on H
         res_hpts = tfsf;
         for (const Src& S : srcs) res_hpts = res_hpts || S.comp <= MFD_HZ;
@@ -899,7 +909,7 @@ class Engine : public HandleBase {
         with_resident_kernel([&](auto k) { MFD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, RES_THREADS<T>, 0)); });
         MFD_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         MFD_CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-        if (per_sm < 1 || !coop) return;
+        if (per_sm < 1 || !coop) return false;
         ResidentParams<T>& p = res_p;
         p.ncell = (int)N;
         // up to one cell per thread of a cluster's blocks: one cluster
@@ -979,9 +989,8 @@ class Engine : public HandleBase {
                     ops.push_back(o);
                 }
                 if (i < srcs.size() && (srcs[i].comp <= MFD_HZ) == (onh != 0)) {
-                    const int64_t* cells = d->srcs[i].cells;
                     const Src& S = srcs[i];
-                    add_list(1, [&](auto&& emit) { for (long long j = 0; j < S.npts; ++j) emit(cells[j], (int)j, 0); });
+                    add_list(1, [&](auto&& emit) { for (long long j = 0; j < S.npts; ++j) emit(res_cells[i][j], (int)j, 0); });
                     ResOp<T> o{};
                     o.kind = S.kind; o.coeff = S.coeff; o.F = F[S.comp]; o.cells = S.cells; o.wave = S.wave; o.amp = S.amp;
                     o.gt = S.gt; o.npts = S.npts;
@@ -994,8 +1003,8 @@ class Engine : public HandleBase {
         p.nmon = mon_p.nmon;
         if (p.nmon)
             add_list(2, [&](auto&& emit) {
-                for (int m = 0; m < d->nmon; ++m)
-                    for (long long j = 0; j < d->mons[m].npts; ++j) emit(d->mons[m].cells[j], m, (int)j);
+                for (int m = 0; m < p.nmon; ++m)
+                    for (long long j = 0; j < mons_host[m].npts; ++j) emit(res_cells[srcs.size() + m][j], m, (int)j);
             });
         int most = 0;   // points of one block
         for (int b = 0; b < res_blocks; ++b) {
@@ -1009,7 +1018,7 @@ class Engine : public HandleBase {
         {   // the grid must still be resident at once with that much shared memory
             int fit = 0;
             with_resident_kernel([&](auto k) { MFD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, RES_THREADS<T>, (size_t)res_smem)); });
-            if ((long long)fit * sms < res_blocks) return;
+            if ((long long)fit * sms < res_blocks) return false;
         }
         if (!all.empty()) {
             const int* da = upload_own(std::move(all));
@@ -1022,7 +1031,20 @@ class Engine : public HandleBase {
         p.dt = dt;
         p.bar = dalloc<unsigned>(1, false);
         p.fault = d_resfault = dalloc<int>(1, false);
-        resident = true;
+        MFD_CK(cudaStreamSynchronize(st));
+        held.clear();
+        return true;
+    }
+
+    // Before the first resident steps.  A model whose lists find no memory takes the separate launches.
+    void make_resident() {
+        try {
+            res_ready = init_resident();
+        } catch (const Error& e) {
+            if (e.code != MFD_ERR_OOM) throw;
+        }
+        resident = res_ready;
+        res_cells.clear();
     }
 
     // Steps it .. it + n - 1 in one launch.
@@ -2061,6 +2083,7 @@ class Engine : public HandleBase {
         if (a != done + 1 || b < a - 1 || b > nt) { err = "steps must be consecutive and within 1..Nt"; return MFD_ERR_INVALID; }
         if (b < a) return MFD_OK;
         MFD_CK(cudaSetDevice(dev));
+        if (resident && !res_ready && !profiling) make_resident();
         // the side streams of the split updates and of the gather, at the first steps that use
         // them (a model stepped by a batch or by the resident kernel never does)
         if (overlap && (use_split || mon_apart) && (!resident || profiling)) make_side_stream();
@@ -2166,7 +2189,7 @@ class Engine : public HandleBase {
         MFD_CK(cudaMemcpyAsync(h_flags + (a - 1), d_flags + (a - 1), (size_t)(b - a + 1) * sizeof(int),
                                cudaMemcpyDeviceToHost, st));
         if (tc_fold) MFD_CK(cudaMemcpyAsync(&h_tcfault, d_tcfault, sizeof(int), cudaMemcpyDeviceToHost, st));
-        if (resident) MFD_CK(cudaMemcpyAsync(&h_resfault, d_resfault, sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (res_ready) MFD_CK(cudaMemcpyAsync(&h_resfault, d_resfault, sizeof(int), cudaMemcpyDeviceToHost, st));
         bounded_sync(st);
         check_fold();
         check_resident();

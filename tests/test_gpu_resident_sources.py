@@ -9,7 +9,8 @@ import pytest
 
 import cases as C
 import maxwellfdtd_b200 as M
-from maxwellfdtd_b200.sources import field_components
+from maxwellfdtd_b200 import _abi
+from maxwellfdtd_b200.sources import comp_index, field_components
 from test_gpu_resident import _outputs, _same
 
 pytestmark = pytest.mark.gpu
@@ -94,3 +95,27 @@ def test_tfsf(n, dtype, mode, gpu_lib):
     model = M.Model(g, M.TFSFSource(data=sol.out["tfsf_record"]), tmax=(steps - 0.5) * dt, pml=5 * D,
                     material=_half_space(-ext[-1] + 6 * D))
     _compare(model, [M.FieldMonitor(plane), M.SpectralMonitor(plane, sum=True)], gpu_lib, dtype, mode)
+
+
+@pytest.mark.parametrize("n", [(1, 1, 2001), (201, 1, 149), (61, 48, 55)])
+def test_point_lists_at_the_first_run_that_uses_them(n, gpu_lib):
+    """A model that is stepped otherwise (profiled here; by a batch) makes no lists: device memory grows
+    at the first resident run only, and runs before it in another way change nothing."""
+    nd, g = _grid(n)
+    src = M.SoftSource(geometry=(0.0,) * nd, waveform=lambda *a: C.pulse(a[-1], t0=3e-15), component="Ex")
+    model = M.Model(g, src, tmax=40.5 * M.model.time_step(g, 0.5), pml=5 * D)
+    b, _ = model.build_desc(np.float32, [M.FieldMonitor((0.0,) * nd)])
+    fields = []
+    for profiled in (0, 9):
+        st = _abi.Stepper(gpu_lib, b, np.float32)
+        made = st.device_bytes()
+        if profiled:
+            st.set_profiling(True)
+            st.run(1, profiled)
+            assert st.device_bytes() == made
+            st.set_profiling(False)
+        st.run(profiled + 1, model.Nt)
+        assert st.device_bytes() > made
+        fields.append([st.read_field(comp_index(c)) for c in field_components(nd)])
+        st.close()
+    assert all(np.array_equal(a, c) for a, c in zip(*fields))
