@@ -431,7 +431,8 @@ MFD_API int mfd_server_handle(mfd_server* s, int64_t id, mfd_handle** h);
 MFD_API int mfd_server_release(mfd_server* s, int64_t id);
 MFD_API int mfd_server_info(mfd_server* s, int64_t* queued, int64_t* running, int64_t* done, int64_t* failed,
                             double* used_bytes, double* peak_used_bytes, int32_t* peak_active);
-/* Device bytes mfd_create would allocate for the descriptor (-1: invalid descriptor). */
+/* Device bytes mfd_create would allocate for the descriptor, and the first read-back after it
+ * (-1: invalid descriptor). */
 MFD_API int64_t mfd_server_footprint(const mfd_desc* desc);
 MFD_API const char* mfd_server_last_error(mfd_server* s);
 
@@ -443,7 +444,7 @@ MFD_API int mfd_set_profiling(mfd_handle* h, int32_t on);
 MFD_API int mfd_kernel_times(const mfd_handle* h, double* ms, int64_t* launches, int32_t n);
 /* Device time of the last mfd_run call (CUDA events around the whole call), in ms. */
 MFD_API int mfd_last_run_ms(const mfd_handle* h, double* ms);
-/* Device bytes held by the handle. */
+/* Device bytes the handle has taken from the device's memory pool. */
 MFD_API int64_t mfd_device_bytes(const mfd_handle* h);
 
 MFD_API const char* mfd_last_error(const mfd_handle* h);

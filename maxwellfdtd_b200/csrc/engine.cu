@@ -20,6 +20,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <stdexcept>
 #include <string>
 #include <thread>
@@ -34,6 +35,7 @@
 #include "batch.cuh"
 #include "resident.cuh"
 #include "geometry.cuh"
+#include "footprint.cuh"
 
 namespace mfd {
 
@@ -499,10 +501,11 @@ class Engine : public HandleBase {
 
     // A model has some 70 device arrays, most of them small, and with many models alive each
     // cudaMallocAsync cost 25 us and more (32 2-D models: 3.5 ms of mfd_create each, 0.5 now).  Arrays
-    // up to ARENA_MAX are cut from chunks that grow with the model; larger ones have their own.
-    static constexpr size_t ARENA_MAX = 4u << 20;
-    char* chunk = nullptr;
-    size_t chunk_left = 0, chunk_next = 256u << 10;
+    // up to ARENA_MAX are cut from blocks that are reserved for several of them at exactly their size,
+    // so that no memory lies idle behind them; others have their own.
+    static constexpr int64_t ARENA_MAX = 4 << 20;
+    char* block = nullptr;
+    size_t block_left = 0;
 
     // n bytes, zeroed; null, with the reason in e, when the device has none.
     void* try_alloc(size_t n, cudaError_t* e = nullptr) {
@@ -514,6 +517,7 @@ class Engine : public HandleBase {
             return nullptr;
         }
         allocs.push_back(p);
+        bytes += (int64_t)n;
         MFD_CK(cudaMemsetAsync(p, 0, n, st));
         return p;
     }
@@ -524,24 +528,40 @@ class Engine : public HandleBase {
         return p;
     }
 
+    // One block for the arrays up to ARENA_MAX that each(f) passes to f.
+    template <typename E_>
+    void reserve(E_&& each) {
+        int64_t n = 0;
+        each([&](int64_t b) { n += b <= ARENA_MAX ? array_room(b) : 0; });
+        if (!n) return;
+        block = (char*)try_alloc((size_t)n);   // without it the arrays have their own, or fail, one by one
+        block_left = block ? (size_t)n : 0;
+    }
+
+    // A block for the arrays made in a scope, beside the one around it.
+    struct BlockScope {
+        Engine& e;
+        char* const block;
+        const size_t left;
+        template <typename E_>
+        BlockScope(Engine& e_, E_&& each) : e(e_), block(e_.block), left(e_.block_left) {
+            e.block_left = 0;
+            e.reserve(each);
+        }
+        ~BlockScope() { e.block = block; e.block_left = left; }
+    };
+
     template <typename U>
     U* dalloc(size_t n, bool state = true) {
-        if (n == 0) n = 1;
-        const size_t b = n * sizeof(U), room = (size_t)round_up((long long)b, 256);
+        const size_t b = std::max<size_t>(n, 1) * sizeof(U), room = (size_t)array_room((int64_t)b);
         void* p;
-        if (b > ARENA_MAX) {
+        if ((int64_t)b > ARENA_MAX || room > block_left) {
             p = raw_alloc(b);
         } else {
-            if (room > chunk_left) {
-                chunk_left = std::max(room, chunk_next);
-                chunk_next = std::min(2 * chunk_next, 2 * ARENA_MAX);
-                chunk = (char*)raw_alloc(chunk_left);
-            }
-            p = chunk;
-            chunk += room;
-            chunk_left -= room;
+            p = block;
+            block += room;
+            block_left -= room;
         }
-        bytes += (int64_t)b;
         if (state) state_bufs.push_back({p, b});
         return (U*)p;
     }
@@ -662,6 +682,7 @@ class Engine : public HandleBase {
         }
         for (int f = 0; f < 6; ++f) bc[f] = d->bc[f];
         Mh0 = (T)d->Mh0; Me0 = (T)d->Me0; Md10 = (T)d->Md10; Md20 = (T)d->Md20;
+        reserve([&](auto&& f) { each_array(d, f); });
         for (int c = 0; c < 9; ++c)
             if (has_comp(c)) F[c] = dalloc<T>(Np);
         Sa = dalloc<T>(Np);
@@ -721,6 +742,11 @@ class Engine : public HandleBase {
                 mbox[4] = first ? bz0[g] : std::min(mbox[4], bz0[g]); mbox[5] = std::max(mbox[5], bz1[g]);
             }
         }
+        std::vector<int64_t> box_cells(nmat, 0);
+        for (int g = 1; g <= nmat; ++g)
+            if (bx1[g] >= 0) box_cells[g - 1] = (int64_t)(bx1[g] - bx0[g] + 1) * (by1[g] - by0[g] + 1) * (bz1[g] - bz0[g] + 1);
+        std::optional<BlockScope> mat_block;
+        mat_block.emplace(*this, [&](auto&& f) { each_material_array(d, box_cells, f); });
         if (any_geom) {
             if (!geom) {   // the caller's map, rows of nx bytes, into rows of px (the padding stays 0)
                 geom = dalloc<uint8_t>((size_t)Np, false);
@@ -777,6 +803,7 @@ class Engine : public HandleBase {
                 }
             }
         }
+        mat_block.reset();
         if (nmat) {
             matMh = upload_own(std::move(mh));
             mats_dev = upload(mats_host.data(), nmat);
@@ -1020,6 +1047,13 @@ class Engine : public HandleBase {
             with_resident_kernel([&](auto k) { MFD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, RES_THREADS<T>, (size_t)res_smem)); });
             if ((long long)fit * sms < res_blocks) return false;
         }
+        BlockScope tables(*this, [&](auto&& f) {
+            if (!all.empty()) f((int64_t)(all.size() * sizeof(int)));
+            if (!ops.empty()) f((int64_t)(ops.size() * sizeof(ResOp<T>)));
+            if (tfsf) f((int64_t)sizeof(tfsf_p));
+            f((int64_t)sizeof(unsigned));   // barrier
+            f((int64_t)sizeof(int));        // its status
+        });
         if (!all.empty()) {
             const int* da = upload_own(std::move(all));
             for (size_t o = 0; o < ops.size(); ++o) { ops[o].off = da + at[o].first; ops[o].list = da + at[o].second; }
@@ -1328,6 +1362,10 @@ class Engine : public HandleBase {
             tfsf_maxlen = std::max(tfsf_maxlen, p.s[i].len);
             if (p.s[i].len >= (1ll << 31)) throw Error(MFD_ERR_INVALID, "TFSF face larger than 2^31 cells");
         }
+        BlockScope arrays(*this, [&](auto&& f) {
+            for (int k = 0; k < narr; ++k)
+                if (nonzero[k]) f((int64_t)clen[k] * nt * (int64_t)sizeof(T));
+        });
         for (int k = 0; k < narr; ++k)
             if (nonzero[k]) p.arr[k] = upload((const T*)d->tfsf.inc[k], (size_t)clen[k] * nt);
         tfsf = n > 0;
@@ -1382,11 +1420,15 @@ class Engine : public HandleBase {
         rec_narr = p.n;
         p.L = layout();
         for (int c = 0; c < 9; ++c) p.F[c] = F[c];
+        auto size = [](const S6& q) { return (long long)(q.x1 - q.x0 + 1) * (q.y1 - q.y0 + 1) * (q.z1 - q.z0 + 1); };
+        BlockScope arrays(*this, [&](auto&& f) {
+            for (const S6& q : v) f((int64_t)size(q) * nt * (int64_t)sizeof(T));
+        });
         for (int i = 0; i < p.n; ++i) {
             RectStmt& s = p.s[i];
             s.comp = v[i].comp; s.x0 = v[i].x0; s.x1 = v[i].x1; s.y0 = v[i].y0; s.y1 = v[i].y1; s.z0 = v[i].z0; s.z1 = v[i].z1;
             s.k = i;
-            s.len = (long long)(s.x1 - s.x0 + 1) * (s.y1 - s.y0 + 1) * (s.z1 - s.z0 + 1);
+            s.len = size(v[i]);
             s.shape = MFD_INC_FULL;
             s.clen = s.len;
             rec_maxlen = std::max(rec_maxlen, s.len);
@@ -2216,27 +2258,30 @@ class Engine : public HandleBase {
     // rows of 244 bytes (nx = 61) came at 5.8 GB/s and rows of 200-500 bytes at 16 GB/s, where
     // rows of 924 bytes reach 44.  Shorter rows are therefore packed on the device (a few us)
     // and copied densely, PACK_BYTES at a time (61 x 48 x 55: 11 arrays and 24 traces 1.28 -> 0.67 ms;
-    // 32 models of 48-128 cells a side: 41 -> 34 ms).  A device without
-    // memory for the buffer still has the strided copy.  noalloc: the caller's read may not take
-    // device memory.
-    static constexpr size_t PACK_ROW = 1024, PACK_BYTES = 8u << 20;
+    // 32 models of 48-128 cells a side: 41 -> 34 ms).  The buffer is made by the first such read and
+    // kept; models whose fields have long rows, but whose map (a byte a cell) has short ones, have
+    // one for that read only.  A device without memory for it still has the strided copy.  noalloc:
+    // the caller's read may not take device memory.
     unsigned char* pack_buf = nullptr;
 
     template <typename U>
     bool copy_packed(const void* dsrc, void* hdst) {   // false: no memory for the buffer, nothing copied
-        const size_t cap = std::min((size_t)N * sizeof(double), PACK_BYTES);   // holds a row of any element type
-        const long long rows = (long long)ny * nz, per = (long long)(cap / sizeof(U)) / nx;
-        if (!pack_buf) {
-            pack_buf = (unsigned char*)try_alloc(cap);
-            if (!pack_buf) return false;
-            bytes += (int64_t)cap;
+        const size_t keep = (size_t)pack_bytes(nx, px, N, sizeof(T)), cap = keep ? keep : std::min((size_t)N * sizeof(U), (size_t)PACK_BYTES);
+        unsigned char* buf = pack_buf;
+        if (!buf && keep) buf = pack_buf = (unsigned char*)try_alloc(keep);
+        if (!buf && !keep && cudaMallocAsync((void**)&buf, cap, st) != cudaSuccess) {
+            cudaGetLastError();
+            buf = nullptr;
         }
+        if (!buf) return false;
+        const long long rows = (long long)ny * nz, per = (long long)(cap / sizeof(U)) / nx;
         for (long long r = 0; r < rows; r += per) {
             const long long n = std::min(per, rows - r) * nx;
-            pack_rows_kernel<U><<<(unsigned)std::min((n + 255) / 256, 148ll * 8), 256, 0, st>>>((const U*)dsrc, (U*)pack_buf, nx, px, r, n);
+            pack_rows_kernel<U><<<(unsigned)std::min((n + 255) / 256, 148ll * 8), 256, 0, st>>>((const U*)dsrc, (U*)buf, nx, px, r, n);
             MFD_CK(cudaGetLastError());
-            MFD_CK(cudaMemcpyAsync((U*)hdst + r * nx, pack_buf, (size_t)n * sizeof(U), cudaMemcpyDeviceToHost, st));
+            MFD_CK(cudaMemcpyAsync((U*)hdst + r * nx, buf, (size_t)n * sizeof(U), cudaMemcpyDeviceToHost, st));
         }
+        if (!keep) MFD_CK(cudaFreeAsync(buf, st));
         return true;
     }
 
@@ -2247,7 +2292,7 @@ class Engine : public HandleBase {
             bounded_sync(st);
             return;
         }
-        const bool packed = !noalloc && (size_t)nx * esize < PACK_ROW &&
+        const bool packed = !noalloc && (int64_t)nx * (int64_t)esize < PACK_ROW &&
                             (esize == 1 ? copy_packed<uint8_t>(dsrc, hdst) : esize == 4 ? copy_packed<uint32_t>(dsrc, hdst)
                                                                                        : copy_packed<uint64_t>(dsrc, hdst));
         if (!packed)

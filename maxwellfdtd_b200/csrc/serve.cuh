@@ -25,24 +25,20 @@
 
 namespace mfd {
 
-// Device bytes mfd_create allocates for a descriptor, before anything is allocated: fields
-// and running sums in the padded layout, the material map and each material's compact state
-// (from the bounding box of its cells), CPML psi slabs and profiles, source tables, TFSF
-// incident arrays (compact layouts counted compact), monitor records, accumulators and the
-// staging ring, the per-step flags, and 64 KiB for small tables.
+// Device bytes that mfd_create allocates for a descriptor (each_array, each_material_array from the
+// bounding boxes of the materials' cells, TFSF incident arrays with compact layouts counted compact)
+// and the read-back buffer that its first read adds, before anything is allocated, and 64 KiB for
+// small tables.
 static int64_t desc_footprint(const mfd_desc* d) {
-    const int64_t T = d->dtype == MFD_F64 ? 8 : 4;
-    const int64_t R = (T == 8 || d->rho_fp64) ? 8 : 4;
+    const int64_t T = desc_tsize(d);
     const int nd = d->ndim;
-    const int64_t px = nd == 1 ? d->nx : (d->nx + 31) / 32 * 32;
-    const int64_t Np = px * d->ny * d->nz;
-    static const int ncomp[4] = {0, 3, 5, 9};
-    const bool ey2 = nd == 2 && d->polarization == MFD_POL_EY;   // Hx, Hz, Dy, Ey
-    int64_t b = ((ey2 ? 4 : ncomp[nd]) + 1) * Np * T + d->nt * 4 + 4;
+    const bool ey2 = nd == 2 && d->polarization == MFD_POL_EY;
+    int64_t b = 0;
+    auto add = [&](int64_t bytes) { b += array_room(bytes); };
+    each_array(d, add);
     const int nmat = d->nmat;
     std::vector<int> x0(nmat + 1, INT32_MAX), x1(nmat + 1, -1), y0(nmat + 1, INT32_MAX), y1(nmat + 1, -1),
         z0(nmat + 1, INT32_MAX), z1(nmat + 1, -1);
-    bool any = false;
     if (d->geometry || (d->nshape > 0 && d->shapes && d->coords[2])) {
         for (int iz = 0; iz < d->nz; ++iz)
             for (int iy = 0; iy < d->ny; ++iy) {
@@ -57,49 +53,20 @@ static int64_t desc_footprint(const mfd_desc* d) {
                             if (shape_covers(d->shapes[k], x, y, d->coords[2][iz])) g = d->shapes[k].material;
                     }
                     if (!g || g > nmat) continue;
-                    any = true;
                     x0[g] = std::min(x0[g], ix); x1[g] = std::max(x1[g], ix);
                     y0[g] = std::min(y0[g], iy); y1[g] = std::max(y1[g], iy);
                     z0[g] = std::min(z0[g], iz); z1[g] = std::max(z1[g], iz);
                 }
             }
     }
-    if (any) b += Np + Np * T;
-    const int nc = ey2 ? 1 : nd;
-    for (int g = 1; g <= nmat; ++g) {
-        const mfd_material& m = d->mats[g - 1];
-        b += T + 512;
-        if (x1[g] < 0) continue;
-        const int64_t bs = (int64_t)(x1[g] - x0[g] + 1) * (y1[g] - y0[g] + 1) * (z1[g] - z0[g] + 1);
-        if (m.nq > 0) b += 2 * m.nq * nc * bs * T;
-        if (m.plasma) b += 2 * (int64_t)m.rate_n * T + 3 * nc * bs * T + 2 * bs * R + bs * T;
-    }
-    for (int f = 0; f < 6; ++f) {
-        const mfd_pml_layer& L = d->pml[f];
-        if (L.nb <= 0) continue;
-        const int axis = f / 2;
-        const bool used = nd == 3 || (nd == 2 && axis != 1) || (nd == 1 && axis == 2);
-        if (!used) continue;
-        b += (int64_t)L.nb * (8 * T) + 2 * (int64_t)L.nb * T;
-        if (nd == 3) {
-            const int64_t cnt = axis == 0 ? (int64_t)L.nb * d->ny * d->nz : axis == 1 ? px * L.nb * d->nz : px * d->ny * L.nb;
-            b += 4 * cnt * T;
-        } else if (nd == 2) {
-            const int64_t cnt = axis == 0 ? (int64_t)L.nb * d->nz : px * L.nb;
-            b += 2 * cnt * T;
-        } else {
-            b += 2 * (int64_t)L.nb * T;
-        }
-    }
-    for (int i = 0; i < d->nsrc; ++i) {
-        const mfd_source& s = d->srcs[i];
-        b += s.npts * 8 + (s.wave ? d->nt * s.npts * 8 : s.npts * 8 + d->nt * 8);
-    }
+    std::vector<int64_t> box_cells(nmat, 0);
+    for (int g = 1; g <= nmat; ++g)
+        if (x1[g] >= 0) box_cells[g - 1] = (int64_t)(x1[g] - x0[g] + 1) * (y1[g] - y0[g] + 1) * (z1[g] - z0[g] + 1);
+    each_material_array(d, box_cells, add);
     // TFSF face arrays: the extents (a, b) of array k of a box, bytes by its layout
-    auto face_bytes = [&](const int* i1, const int* i2, const int32_t* shape) {
+    auto face_arrays = [&](const int* i1, const int* i2, const int32_t* shape) {
         const int64_t Nx = i2[0] - i1[0], Ny = i2[1] - i1[1], Nz = i2[2] - i1[2];
         const int narr = nd == 3 ? 24 : nd == 2 ? 8 : 4;
-        int64_t sum = 0;
         for (int k = 0; k < narr; ++k) {
             int64_t a = 1, bb = 1;
             if (nd == 2) a = (k < 4 ? Nz : Nx) + (ey2 ? 1 : 0);   // the second field set spans the nodes
@@ -111,25 +78,12 @@ static int64_t desc_footprint(const mfd_desc* d) {
                 else { a = p ? Nx + 1 : Nx; bb = p ? Ny : Ny + 1; }
             }
             const int sh = shape ? shape[k] : MFD_INC_FULL;
-            sum += (sh == MFD_INC_ALONG_B ? bb : sh == MFD_INC_ALONG_A ? a : sh == MFD_INC_UNIFORM ? 1 : a * bb) * d->nt * T;
+            add((sh == MFD_INC_ALONG_B ? bb : sh == MFD_INC_ALONG_A ? a : sh == MFD_INC_UNIFORM ? 1 : a * bb) * d->nt * T);
         }
-        return sum;
     };
-    if (d->tfsf.enabled) b += face_bytes(d->tfsf.i1, d->tfsf.i2, d->tfsf.shape);
-    if (d->tfsf_record) b += face_bytes(d->rec_i1, d->rec_i2, nullptr);
-    static const int ncm[4] = {0, 2, 3, 6};
-    int64_t ring_vals = 0;
-    for (int i = 0; i < d->nmon; ++i) {
-        const mfd_monitor& m = d->mons[i];
-        b += m.npts * 4 + 64;
-        if (m.kind == MFD_MON_FIELD) b += ncm[nd] * d->nt * (m.sum ? 1 : m.npts) * T;
-        else b += ncm[nd] * (int64_t)m.nw * (m.sum ? 1 : m.npts) * 16 + d->nt * (int64_t)m.nw * 16;
-        if (m.kind != MFD_MON_FIELD || m.sum) ring_vals += ncm[nd] * m.npts;
-    }
-    if (ring_vals) {
-        const int64_t k = std::max<int64_t>(1, std::min<int64_t>(64, (512ll << 20) / (T * ring_vals)));
-        b += k * ring_vals * T;
-    }
+    if (d->tfsf.enabled) face_arrays(d->tfsf.i1, d->tfsf.i2, d->tfsf.shape);
+    if (d->tfsf_record) face_arrays(d->rec_i1, d->rec_i2, nullptr);
+    b += pack_bytes(d->nx, padded_nx(d), (int64_t)d->nx * d->ny * d->nz, T);
     return b + (64 << 10);
 }
 

@@ -35,29 +35,36 @@ from . import _abi
 BATCH_3D_MAX_CELLS = 1 << 20   # 3-D requests up to this many cells join the batch
 
 _NCOMP = {1: 3, 2: 5, 3: 9}
-_NCOMP_E = {1: 1, 2: 2, 3: 3}
 _NCOMP_MON = {1: 2, 2: 3, 3: 6}
+_PACK_ROW, _PACK_BYTES = 1024, 8 << 20   # csrc/footprint.cuh
 
 
 def footprint(builder, model, dtype=np.float32):
-    """Device bytes mfd_create allocates for this descriptor: the fields and running sums
-    in the padded layout, the material map and compact material state, CPML psi slabs,
-    source, TFSF and monitor tables, per-step flags.  Used for admission (before anything
-    is allocated)."""
+    """Device bytes that mfd_create allocates for this descriptor (the fields and running sums in
+    the padded layout, the material map and compact material state, CPML psi slabs, source, TFSF
+    and monitor tables, per-step flags, each rounded up to 256 bytes) and the read-back buffer that
+    its first read adds.  Used for admission (before anything is allocated)."""
     d = builder.desc
     T = np.dtype(dtype).itemsize
     R = 8 if (T == 8 or d.rho_fp64) else 4
     nd = d.ndim
     px = d.nx if nd == 1 else -(-d.nx // 32) * 32
     Np = px * d.ny * d.nz
-    b = (_NCOMP[nd] + 1) * Np * T + d.nt * 4 + 4
+
+    def room(*sizes):
+        return sum(max(1, -(-int(n) // 256)) * 256 for n in sizes)
+
+    b = (_NCOMP[nd] + 1) * room(Np * T) + room(d.nt * 4)
     geom = np.asarray(model.geometry)
     if np.any(geom):
-        b += Np + Np * T
-    nc = _NCOMP_E[nd]
+        b += room(Np, Np * T)
+    if d.nmat:
+        b += room(d.nmat * T, d.nmat * 1024)
+    nc = nd
     for g in range(1, d.nmat + 1):
         m = d.mats[g - 1]
-        b += T + 512
+        if m.plasma:
+            b += 2 * room(m.rate_n * T)
         idx = np.nonzero(geom == g)
         if len(idx[0]) == 0:
             continue
@@ -65,9 +72,9 @@ def footprint(builder, model, dtype=np.float32):
         for ax in idx:
             bsize *= int(ax.max() - ax.min() + 1)
         if m.nq > 0:
-            b += 2 * m.nq * nc * bsize * T
+            b += room(2 * m.nq * nc * bsize * T)
         if m.plasma:
-            b += 2 * m.rate_n * T + 3 * nc * bsize * T + 2 * bsize * R + bsize * T
+            b += room(2 * nc * bsize * T, nc * bsize * T, bsize * R, bsize * R, bsize * T)
     for f in range(6):
         L = d.pml[f]
         if L.nb <= 0:
@@ -76,36 +83,40 @@ def footprint(builder, model, dtype=np.float32):
         used = nd == 3 or (nd == 2 and axis != 1) or (nd == 1 and axis == 2)
         if not used:
             continue
-        b += L.nb * (8 * T) + 2 * L.nb * T
+        b += room(L.nb * 8 * T, L.nb * T, L.nb * T)
         if nd == 3:
             cnt = (L.nb * d.ny * d.nz, px * L.nb * d.nz, px * d.ny * L.nb)[axis]
-            b += 4 * cnt * T
+            b += 4 * room(cnt * T)
         elif nd == 2:
             cnt = L.nb * d.nz if axis == 0 else px * L.nb
-            b += 2 * cnt * T
+            b += 2 * room(cnt * T)
         else:
-            b += 2 * L.nb * T
+            b += 2 * room(L.nb * T)
     for i in range(d.nsrc):
         s = d.srcs[i]
-        b += s.npts * 8 + (d.nt * s.npts * 8 if s.wave else s.npts * 8 + d.nt * 8)
+        b += room(s.npts * 8) + (room(d.nt * s.npts * 8) if s.wave else room(s.npts * 8, d.nt * 8))
     if d.tfsf.enabled:
-        b += sum(a.nbytes for a in builder.keep if isinstance(a, np.ndarray) and a.ndim == 2 and a.shape[0] == d.nt
+        b += sum(room(a.nbytes) for a in builder.keep if isinstance(a, np.ndarray) and a.ndim == 2 and a.shape[0] == d.nt
                  and a.dtype == np.dtype(dtype))
     ring_vals = 0
     ncm = _NCOMP_MON[nd]
     for i in range(d.nmon):
         mo = d.mons[i]
-        b += mo.npts * 4 + 64
-        if mo.kind == _abi.MFD_MON_FIELD:
-            b += ncm * d.nt * (1 if mo.sum else mo.npts) * T
-        else:
-            b += ncm * mo.nw * (1 if mo.sum else mo.npts) * 16 + d.nt * mo.nw * 16
         if mo.kind != _abi.MFD_MON_FIELD or mo.sum:
             ring_vals += ncm * mo.npts
-    if ring_vals:
-        ring_k = max(1, min(64, (512 << 20) // (T * ring_vals)))
-        b += ring_k * ring_vals * T
-    return int(b) + (64 << 10)   # small tables (descriptors, divisor checks) and rounding
+    ring_k = max(1, min(64, (512 << 20) // (T * ring_vals))) if ring_vals else 0
+    for i in range(d.nmon):
+        mo = d.mons[i]
+        b += room(mo.npts * 4) + 64
+        if mo.kind == _abi.MFD_MON_FIELD:
+            b += room(ncm * d.nt * (1 if mo.sum else mo.npts) * T)
+        else:
+            b += room(ncm * mo.nw * (1 if mo.sum else mo.npts) * 16, d.nt * mo.nw * 16)
+        if mo.kind != _abi.MFD_MON_FIELD or mo.sum:
+            b += room(ring_k * ncm * mo.npts * T)
+    if d.nx != px and d.nx * T < _PACK_ROW:   # read-backs of short rows
+        b += min(max(d.nx * d.ny * d.nz * T, 8 * d.nx), _PACK_BYTES)
+    return int(b) + (64 << 10)   # small tables (descriptors, divisor checks, shapes and coordinates)
 
 
 class Request:
