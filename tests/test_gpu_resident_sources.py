@@ -119,3 +119,31 @@ def test_point_lists_at_the_first_run_that_uses_them(n, gpu_lib):
         fields.append([st.read_field(comp_index(c)) for c in field_components(nd)])
         st.close()
     assert all(np.array_equal(a, c) for a, c in zip(*fields))
+
+
+# around one block (128 cells), one cluster (8 blocks of 640 or 512 threads), one round of 148 blocks, and
+# the largest models that step so; whether they do
+THRESHOLDS = [("float32", (1, 1, 128), True), ("float32", (1, 1, 129), True), ("float32", (1, 1, 5120), True),
+              ("float32", (1, 1, 5121), True), ("float32", (64, 1, 80), True), ("float32", (61, 1, 84), True),
+              ("float32", (320, 1, 296), True), ("float32", (313, 1, 303), True), ("float32", (1000, 1, 1000), True),
+              ("float32", (1001, 1, 1000), False), ("float32", (100, 100, 75), True), ("float32", (100, 100, 76), False),
+              ("float64", (1, 1, 128), True), ("float64", (1, 1, 129), True), ("float64", (1, 1, 4096), True),
+              ("float64", (1, 1, 4097), True), ("float64", (256, 1, 296), True), ("float64", (257, 1, 295), True),
+              ("float64", (1000, 1, 1000), True), ("float64", (1001, 1, 1000), False), ("float64", (100, 100, 75), True),
+              ("float64", (100, 100, 76), False)]
+
+
+@pytest.mark.parametrize("dtype,n,small", THRESHOLDS)
+def test_sizes_around_the_thresholds(dtype, n, small, gpu_lib):
+    nd, g = _grid(n)
+    dt = np.dtype(dtype).type
+    at = tuple(0.11 * float(a[-1]) for a in ((g.x, g.y, g.z) if nd == 3 else (g.x, g.z) if nd == 2 else (g.z,)))
+    src = M.SoftSource(geometry=at, waveform=lambda *a: C.pulse(a[-1], t0=3e-15), component="Ex")
+    plane = lambda *c: np.abs(c[-1] - at[-1]) < 0.6 * D
+    mons = [M.FieldMonitor(at), M.SpectralMonitor(plane, sum=True)]
+    model = M.Model(g, src, tmax=40.5 * M.model.time_step(g, 0.5), pml=5 * D, material=_half_space(at[-1]))
+    ref, n2 = _outputs(model, gpu_lib, dt, mons, "exact", True, [])
+    got, n1 = _outputs(model, gpu_lib, dt, mons, "exact", False, [5])
+    assert (n1 < n2 / 4) == small
+    _same(ref, got)
+    assert np.abs(got["Ex"]).max() > 0
