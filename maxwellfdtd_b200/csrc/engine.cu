@@ -1634,18 +1634,14 @@ class Engine : public HandleBase {
     }
     template <bool MATH, int FAST>
     void launch_H_t(const HParams<T>& p) {
-        if constexpr (sizeof(T) == 4 && FAST != DIV_IEEE) {
-            if (quad2d()) {
-                h2d_quad_kernel<MATH, FAST><<<dim3((nx + 127) / 128, (nz + Q_TY - 1) / Q_TY), dim3(32, Q_TY), 0, st>>>(p, kappa_one);
-                return;
-            }
-        }
         if (ndim == 3) {
             dim3 blk(bx3, by3), grd((nx + bx3 - 1) / bx3, (ny + by3 - 1) / by3, (nz + zc3 - 1) / zc3);
             h3d_kernel<T, MATH, FAST><<<grd, blk, 0, st>>>(p, zc3);
         } else if (ndim == 2) {
             dim3 blk(32, 8), grd((nx + 31) / 32, (nz + 7) / 8);
             if (ey2) h2e_kernel<T, MATH, FAST><<<grd, blk, 0, st>>>(p);
+            else if constexpr (sizeof(T) == 4 && FAST != DIV_IEEE)   // quad2d()
+                h2d_quad_kernel<MATH, FAST><<<dim3((nx + 127) / 128, (nz + Q_TY - 1) / Q_TY), dim3(32, Q_TY), 0, st>>>(p, kappa_one);
             else h2d_kernel<T, MATH, FAST><<<grd, blk, 0, st>>>(p);
         } else {
             dim3 blk(256), grd((nz + 255) / 256);
@@ -1891,21 +1887,25 @@ class Engine : public HandleBase {
     }
 
     template <bool MAT, int FAST>
-    void launch_E_t(const EParams<T, R>& p, int cur) {
-        if constexpr (sizeof(T) == 4 && FAST != DIV_IEEE) {
-            if (quad2d()) {
-                const dim3 grd((nx + 127) / 128, (nz + Q_TY - 1) / Q_TY), blk(32, Q_TY);
-                if (MAT && !response_mats.empty() && quad_resp()) e2d_quad_kernel<R, MAT, FAST, true><<<grd, blk, 0, st>>>(p, kappa_one, cur);
-                else e2d_quad_kernel<R, MAT, FAST, false><<<grd, blk, 0, st>>>(p, kappa_one, cur);
+    void launch_e2d_quad(const EParams<T, R>& p, int cur) {
+        const dim3 grd((nx + 127) / 128, (nz + Q_TY - 1) / Q_TY), blk(32, Q_TY);
+        if constexpr (MAT) {
+            if (!response_mats.empty() && quad_resp()) {
+                e2d_quad_kernel<R, true, FAST, true><<<grd, blk, 0, st>>>(p, kappa_one, cur);
                 return;
             }
         }
+        e2d_quad_kernel<R, MAT, FAST, false><<<grd, blk, 0, st>>>(p, kappa_one, cur);
+    }
+    template <bool MAT, int FAST>
+    void launch_E_t(const EParams<T, R>& p, int cur) {
         if (ndim == 3) {
             dim3 blk(bx3, by3), grd((nx + bx3 - 1) / bx3, (ny + by3 - 1) / by3, (nz + zc3 - 1) / zc3);
             e3d_kernel<T, R, MAT, FAST><<<grd, blk, 0, st>>>(p, zc3);
         } else if (ndim == 2) {
             dim3 blk(32, 8), grd((nx + 31) / 32, (nz + 7) / 8);
             if (ey2) e2e_kernel<T, R, MAT, FAST><<<grd, blk, 0, st>>>(p);
+            else if constexpr (sizeof(T) == 4 && FAST != DIV_IEEE) launch_e2d_quad<MAT, FAST>(p, cur);   // quad2d()
             else e2d_kernel<T, R, MAT, FAST><<<grd, blk, 0, st>>>(p);
         } else {
             dim3 blk(256), grd((nz + 255) / 256);

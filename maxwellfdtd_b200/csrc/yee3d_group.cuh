@@ -16,31 +16,22 @@ namespace mfd {
 
 template <int W>
 __device__ __forceinline__ void g_load(const float* p, float (&v)[W]) {
-    if constexpr (W == 4) {
-        const float4 a = *reinterpret_cast<const float4*>(p);
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    } else {
-        const float2 a = *reinterpret_cast<const float2*>(p);
-        v[0] = a.x; v[1] = a.y;
-    }
+    static_assert(W == 2, "the accesses are of two cells");
+    const float2 a = *reinterpret_cast<const float2*>(p);
+    v[0] = a.x; v[1] = a.y;
 }
 // nv: how many of the cells lie in the row (the padding behind it stays zero).
 template <int W>
 __device__ __forceinline__ void g_store(float* p, const float (&v)[W], int nv) {
-    if (nv == W) {
-        if constexpr (W == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-        else *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
-    } else {
-#pragma unroll
-        for (int j = 0; j < W - 1; ++j)
-            if (j < nv) p[j] = v[j];
-    }
+    static_assert(W == 2, "the accesses are of two cells");
+    if (nv == W) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+    else p[0] = v[0];
 }
 // The material indices of a group, packed (byte j: cell j).
 template <int W>
 __device__ __forceinline__ unsigned g_geom(const uint8_t* p) {
-    if constexpr (W == 4) return *reinterpret_cast<const unsigned*>(p);
-    else return *reinterpret_cast<const unsigned short*>(p);
+    static_assert(W == 2, "the accesses are of two cells");
+    return *reinterpret_cast<const unsigned short*>(p);
 }
 
 // One CPML face of axis AX (0 x, 1 y, 2 z) of a group: the psi pair P, P + 1 of derivatives da, db
