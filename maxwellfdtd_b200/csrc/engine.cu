@@ -500,7 +500,7 @@ class Engine : public HandleBase {
     std::vector<std::pair<void*, size_t>> state_bufs;
 
     // A model has some 70 device arrays, most of them small, and with many models alive each
-    // cudaMallocAsync cost 25 us and more (32 2-D models: 3.5 ms of mfd_create each, 0.5 now).  Arrays
+    // cudaMallocAsync cost 25 us and more (32 2-D models: 3.5 ms of mfd_create each, 0.36 now).  Arrays
     // up to ARENA_MAX are cut from blocks that are reserved for several of them at exactly their size,
     // so that no memory lies idle behind them; others have their own.
     static constexpr int64_t ARENA_MAX = 4 << 20;
@@ -867,6 +867,8 @@ class Engine : public HandleBase {
         h_flags_v.assign((size_t)nt, 0);
         h_flags = h_flags_v.data();
         init_split();
+        res_hpts = tfsf;
+        for (const Src& S : srcs) res_hpts = res_hpts || S.comp <= MFD_HZ;
         resident = resident_model();
         if (resident) {
             for (int i = 0; i < d->nsrc; ++i) res_cells.emplace_back(d->srcs[i].cells, d->srcs[i].cells + d->srcs[i].npts);
@@ -878,14 +880,36 @@ class Engine : public HandleBase {
     }
 
     // ---- resident steps (resident.cuh) -------------------------------------------------
-    // Cells up to which the resident steps are the faster way (us per step, separate launches
-    // against resident, dispersive model with CPML, one point source and four monitors):
-    //   1-D, any: 3 000 cells 24.3 / 4.5 (one cluster: 3.9), 60 000 35.0 / 5.0;
-    //   2-D float 301 x 300 22.8 / 6.8, 701 x 700 27.7 / 18.0, 1101 x 1100 36.9 / 34.0;
-    //   2-D double 301 x 300 24.6 / 9.7, 901 x 900 35.9 / 31.7, 1101 x 1100 48.4 / 49.2;
-    //   3-D float 46 x 45 x 44 36.7 / 9.0, 91 x 90 x 89 54.0 / 43.3 (tolerance mode 43 / 36.5);
-    //   3-D double 46 x 45 x 44 37.5 / 12.7, 91 x 90 x 89 69.8 / 57.4, 100^3 82 / 102.
-    static long long resident_limit(int nd) { return nd == 3 ? 750000 : 1000000; }
+    // Cells up to which a model takes the resident steps: near where both ways take the same time (us per
+    // step, resident / separate launches; light: no map, map: plain dielectrics, response: a medium whose
+    // E has a response; H points: a TFSF source, whose statements on H wait for the second barrier):
+    //   1-D, any: 3 000 cells 3.8 / 25.1, 60 000 5.1 / 35.5.
+    //   3-D float, any: 728 000 cells light 33.2 / 45.0, map with TFSF 39.8 / 43.9 (tolerance mode 40.3 / 41.8).
+    //   3-D double: the cells' FP64 instructions at 8 warps per SM come to count.  Exact: light 593 000 39.3 /
+    //     43.7, 728 000 49.5 / 47.0; response 728 000 56.9 / 61.5.  Tolerance mode, whose separate launches
+    //     spend fewer instructions: light 593 000 33.7 / 35.5, 728 000 42.4 / 38.5; light with TFSF 300 000
+    //     22.7 / 25.6, 402 000 28.9 / 25.7, map 300 000 22.2 / 27.8, 402 000 29.4 / 27.8; response 593 000 42.3
+    //     / 44.9, 728 000 53.1 / 46.6.
+    //   2-D float, first field set (separate: four cells per thread): light 600 000 19.2 / 19.4, 800 000 22.9 /
+    //     20.6, map 600 000 20.2 / 24.6, 700 000 22.3 / 20.6, 800 000 24.0 / 23.6.
+    //   2-D otherwise: light exact 600 000 19.0 / 20.2 (double 19.7 / 22.6), 800 000 22.9 / 21.3 (25.7 / 24.7);
+    //     light, tolerance mode, double 700 000 23.3 / 24.4, 899 000 27.6 / 25.2, float 997 000 24.2 / 25.7;
+    //     map, double exact 800 000 28.8 / 29.5, 997 000 35.4 / 32.8; map otherwise 997 000 27.5 / 28.0 and better.
+    //   2-D, light with TFSF: 499 000 float 18.0 / 16.9 (tolerance mode 15.8 / 16.5), double 20.7 / 21.4, 600 000
+    //     21.0 / 19.8, 23.6 / 22.7.
+    long long resident_limit() const {
+        const bool dbl = sizeof(T) == 8, response = !response_mats.empty();
+        if (ndim == 1) return 1000000;
+        if (ndim == 3) {
+            if (!dbl) return 750000;
+            if (response) return recip ? 650000 : 750000;
+            return recip && (res_hpts || any_geom) ? 350000 : 650000;
+        }
+        if (res_hpts && !any_geom) return 500000;
+        if (!dbl && !ey2) return 650000;
+        if (!any_geom) return !recip ? 650000 : dbl ? 800000 : 1000000;
+        return dbl && !recip && !response ? 850000 : 1000000;
+    }
 
     template <typename F_>
     void with_resident_kernel(F_&& f) {
@@ -915,7 +939,7 @@ class Engine : public HandleBase {
     // transcendental code, and compute-bound), more than three poles, divisors that failed the check,
     // CPML layers that overlap, more than RES_MAXOPS sources.
     bool resident_model() const {
-        if (!std::is_same<R, double>::value || !overlap || record || any_plasma || N > resident_limit(ndim)) return false;
+        if (!std::is_same<R, double>::value || !overlap || record || any_plasma || N > resident_limit()) return false;
         if (!recip && !fastdiv) return false;
         // an explicit choice of the 3-D kernels keeps them
         if (ndim == 3 && (std::getenv("MFD_KERNEL3D") || std::getenv("MFD_CORE_ASYNC"))) return false;
@@ -930,8 +954,6 @@ class Engine : public HandleBase {
     // so: a model that a batch steps needs neither.  False: the grid would not be resident at once.
     bool init_resident() {
         const int nops = (int)srcs.size() + (tfsf ? 2 : 0);   // the TFSF replay: on E and D, and on H
-        res_hpts = tfsf;
-        for (const Src& S : srcs) res_hpts = res_hpts || S.comp <= MFD_HZ;
         int per_sm = 0, sms = 0, coop = 0;
         with_resident_kernel([&](auto k) { MFD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, RES_THREADS<T>, 0)); });
         MFD_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -17,8 +17,8 @@ pytestmark = pytest.mark.gpu
 
 D = 50e-9
 # threads of a block at most: 640 (float), 512 (double); a cluster of 8 blocks up to 5120 / 4096 cells
-SIZES = [(1, 1, 128), (1, 1, 129), (1, 1, 4097), (1, 1, 5121), (1, 1, 60013), (64, 1, 64), (331, 1, 577), (997, 1, 1001),
-         (16, 16, 20), (67, 61, 59), (90, 91, 91)]
+SIZES = [(1, 1, 128), (1, 1, 129), (1, 1, 4097), (1, 1, 5121), (1, 1, 60013), (64, 1, 64), (331, 1, 577), (806, 1, 805),
+         (16, 16, 20), (67, 61, 59), (90, 91, 79)]
 
 
 def _grid(n):
@@ -121,29 +121,46 @@ def test_point_lists_at_the_first_run_that_uses_them(n, gpu_lib):
     assert all(np.array_equal(a, c) for a, c in zip(*fields))
 
 
-# around one block (128 cells), one cluster (8 blocks of 640 or 512 threads), one round of 148 blocks, and
-# the largest models that step so; whether they do
-THRESHOLDS = [("float32", (1, 1, 128), True), ("float32", (1, 1, 129), True), ("float32", (1, 1, 5120), True),
-              ("float32", (1, 1, 5121), True), ("float32", (64, 1, 80), True), ("float32", (61, 1, 84), True),
-              ("float32", (320, 1, 296), True), ("float32", (313, 1, 303), True), ("float32", (1000, 1, 1000), True),
-              ("float32", (1001, 1, 1000), False), ("float32", (100, 100, 75), True), ("float32", (100, 100, 76), False),
-              ("float64", (1, 1, 128), True), ("float64", (1, 1, 129), True), ("float64", (1, 1, 4096), True),
-              ("float64", (1, 1, 4097), True), ("float64", (256, 1, 296), True), ("float64", (257, 1, 295), True),
-              ("float64", (1000, 1, 1000), True), ("float64", (1001, 1, 1000), False), ("float64", (100, 100, 75), True),
-              ("float64", (100, 100, 76), False)]
+# around one block (128 cells), one cluster (8 blocks of 640 or 512 threads) and one round of 148 blocks
+SMALL = [("float32", n) for n in ((1, 1, 128), (1, 1, 129), (1, 1, 5120), (1, 1, 5121), (64, 1, 80), (61, 1, 84), (320, 1, 296), (313, 1, 303))] + \
+        [("float64", n) for n in ((1, 1, 128), (1, 1, 129), (1, 1, 4096), (1, 1, 4097), (256, 1, 296), (257, 1, 295))]
+# the largest models that step so and the next: (type, mode, field set, medium, H source, the larger of the two sizes)
+LIMITS = [("float32", "exact", "Hy", "response", False, (807, 1, 806)), ("float32", "fast", "Hy", "map", True, (807, 1, 806)),
+          ("float32", "exact", "Hy", "light", True, (709, 1, 706)), ("float64", "fast", "Hy", "light", True, (709, 1, 706)),
+          ("float64", "exact", "Hy", "light", False, (807, 1, 806)), ("float64", "fast", "Ey", "light", False, (895, 1, 894)),
+          ("float32", "fast", "Ey", "light", False, (1001, 1, 1000)), ("float32", "exact", "Ey", "map", False, (1001, 1, 1000)),
+          ("float64", "exact", "Hy", "map", False, (922, 1, 922)), ("float64", "exact", "Hy", "response", False, (1001, 1, 1000)),
+          ("float32", "exact", "", "map", True, (100, 100, 76)), ("float64", "exact", "", "response", False, (100, 100, 76)),
+          ("float64", "exact", "", "map", True, (100, 100, 66)), ("float64", "fast", "", "response", True, (100, 100, 66)),
+          ("float64", "fast", "", "light", False, (100, 100, 66)), ("float64", "fast", "", "light", True, (100, 100, 36)),
+          ("float64", "fast", "", "map", False, (100, 100, 36))]
 
 
-@pytest.mark.parametrize("dtype,n,small", THRESHOLDS)
-def test_sizes_around_the_thresholds(dtype, n, small, gpu_lib):
+def _threshold(dtype, mode, pol, medium, hsrc, n, small, lib):
     nd, g = _grid(n)
     dt = np.dtype(dtype).type
     at = tuple(0.11 * float(a[-1]) for a in ((g.x, g.y, g.z) if nd == 3 else (g.x, g.z) if nd == 2 else (g.z,)))
-    src = M.SoftSource(geometry=at, waveform=lambda *a: C.pulse(a[-1], t0=3e-15), component="Ex")
+    src = [M.SoftSource(geometry=at, waveform=lambda *a: C.pulse(a[-1], t0=3e-15), component="Ey" if pol == "Ey" else "Ex")]
+    if hsrc:
+        src.append(M.SoftSource(geometry=at, waveform=lambda *a: 1e-3 * C.pulse(a[-1], t0=2e-15), component="Hy"))
     plane = lambda *c: np.abs(c[-1] - at[-1]) < 0.6 * D
     mons = [M.FieldMonitor(at), M.SpectralMonitor(plane, sum=True)]
-    model = M.Model(g, src, tmax=40.5 * M.model.time_step(g, 0.5), pml=5 * D, material=_half_space(at[-1]))
-    ref, n2 = _outputs(model, gpu_lib, dt, mons, "exact", True, [])
-    got, n1 = _outputs(model, gpu_lib, dt, mons, "exact", False, [5])
+    mat = {"light": None, "map": M.Material(geometry=lambda *c: c[-1] > at[-1], eps=2.25), "response": _half_space(at[-1])}[medium]
+    model = M.Model(g, src, tmax=40.5 * M.model.time_step(g, 0.5), pml=5 * D, material=mat, polarization=pol or "Hy")
+    ref, n2 = _outputs(model, lib, dt, mons, mode, True, [])
+    got, n1 = _outputs(model, lib, dt, mons, mode, False, [5])
     assert (n1 < n2 / 4) == small
     _same(ref, got)
-    assert np.abs(got["Ex"]).max() > 0
+    assert np.abs(got["Ey" if pol == "Ey" else "Ex"]).max() > 0
+
+
+@pytest.mark.parametrize("dtype,n", SMALL)
+def test_sizes_around_blocks_and_clusters(dtype, n, gpu_lib):
+    _threshold(dtype, "exact", "", "response", False, n, True, gpu_lib)
+
+
+@pytest.mark.parametrize("dtype,mode,pol,medium,hsrc,n", LIMITS)
+def test_largest_resident_models(dtype, mode, pol, medium, hsrc, n, gpu_lib):
+    below = n[:2] + (n[2] - 1,) if n[1] > 1 else (n[0] - 1, 1, n[2])
+    _threshold(dtype, mode, pol, medium, hsrc, n, False, gpu_lib)
+    _threshold(dtype, mode, pol, medium, hsrc, below, True, gpu_lib)
