@@ -27,10 +27,10 @@
 // arithmetic -> store of about 1 us per half-step for one cell per thread; from about 500 cells
 // per SM on the instructions of the cells.  Up to one cell per thread of eight blocks the grid is
 // one thread-block cluster with the hardware's barrier (2 001 cells: 4.5 us per step with the grid
-// barrier, 3.85 so).  Measured per step, separate launches / resident: 2 001 cells 1-D double
-// 20.5 / 3.85 us, 201 x 149 float 15.3 / 5.2, 61 x 48 x 55 float 42.7 /
-// 12.2, 701 x 513 double 25.2 / 14.9.  The engine's resident_limit says up to which size it is
-// used.
+// barrier, 3.7 so).  Measured per step, separate launches / resident: 2 001 cells 1-D double
+// 20.5 / 3.7 us, 201 x 149 float 15.3 / 5.5, 61 x 48 x 55 float 42.7 / 11.8, 701 x 513 double 25.2 /
+// 15.7; the smallest ones vary by 4 % either way with where the pool places their arrays.  The engine's
+// resident_limit says up to which size it is used.
 #pragma once
 
 #include "aux.cuh"
